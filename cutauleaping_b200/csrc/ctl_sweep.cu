@@ -37,67 +37,11 @@
 
 #include "ctl_internal.h"
 
+#include "ctl_fitness.cuh"
 #include "ctl_sweep_dev.cuh"
 #include "ctl_tiny.h"
 
 namespace ctl {
-namespace dev {
-
-// calculateFitness (tau.cu:3324-3408): one thread per parameter set.
-__global__ void fitness_kernel(const uint32_t* __restrict__ samples, const uint32_t* __restrict__ target,
-                               const uint8_t* __restrict__ swarm, double* __restrict__ fitness,
-                               uint32_t threads, uint32_t nsets, uint32_t p_rep, uint32_t ns,
-                               uint32_t so, uint32_t E, uint32_t REP) {
-    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
-    if (tid >= nsets) return;
-    const uint32_t b = tid / threads, t = tid % threads;
-    const uint32_t ex = swarm[tid];
-    float sub = 0.0f;
-    for (uint32_t c = 0; c < ns; c++) {
-        for (uint32_t s = 0; s < so; s++) {
-            double acc = 0.0;
-            for (uint32_t par = 0; par < p_rep; par++) {
-                const size_t gid = (size_t)(b * p_rep + par) * threads + t;
-                acc = acc + (double)samples[(gid * ns + c) * so + s];
-            }
-            acc = acc / (double)p_rep;
-            for (uint32_t e = 0; e < REP; e++) {
-                const int tgt = (int)target[((size_t)(c * E + ex) * REP + e) * so + s];
-                double dist = fabs((double)tgt - acc);
-                if (tgt != 0) dist = dist / (double)tgt;
-                sub = (float)((double)sub + dist);
-            }
-        }
-    }
-    fitness[tid] = ((1.0 / (double)ns) * (1.0 / (double)so)) * (double)sub;
-}
-
-// The same from per-set sample sums (fitness mode of the sweep): the
-// reference's FP64 running sum of p_rep integer samples is exact, so it
-// equals the integer sum converted once; the rest is calculateFitness.
-__global__ void fitness_sums_kernel(const unsigned long long* __restrict__ sums, const uint32_t* __restrict__ target,
-                                    const uint8_t* __restrict__ swarm, double* __restrict__ fitness,
-                                    uint32_t nsets, uint32_t p_rep, uint32_t ns, uint32_t so, uint32_t E,
-                                    uint32_t REP) {
-    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
-    if (tid >= nsets) return;
-    const uint32_t ex = swarm[tid];
-    float sub = 0.0f;
-    for (uint32_t c = 0; c < ns; c++) {
-        for (uint32_t s = 0; s < so; s++) {
-            const double acc = (double)sums[((size_t)tid * ns + c) * so + s] / (double)p_rep;
-            for (uint32_t e = 0; e < REP; e++) {
-                const int tgt = (int)target[((size_t)(c * E + ex) * REP + e) * so + s];
-                double dist = fabs((double)tgt - acc);
-                if (tgt != 0) dist = dist / (double)tgt;
-                sub = (float)((double)sub + dist);
-            }
-        }
-    }
-    fitness[tid] = ((1.0 / (double)ns) * (1.0 / (double)so)) * (double)sub;
-}
-
-}  // namespace dev
 
 // ---------------------------------------------------------------------------
 // Host launch side
@@ -1431,6 +1375,15 @@ extern "C" void ctl_graph_free(ctl_graph* g) {
     delete g;
 }
 
+static ctl_status launch_fitness(const fit::Args& a, cudaStream_t s) {
+    int dev = 0;
+    CTL_CUDA(cudaGetDevice(&dev));
+    DevAttr da;
+    const bool known = device_attr(dev, da) == CTL_OK;
+    CTL_CUDA(fit::launch(a, fit::shape_for(a, known ? da.sm_count : 148), s));
+    return CTL_OK;
+}
+
 extern "C" ctl_status ctl_fitness_device(const uint32_t* d_samples, uint32_t ns, uint32_t s_out,
                                          const uint32_t* d_target, const uint8_t* d_experiment,
                                          uint32_t experiments, uint32_t repetitions, uint32_t threads,
@@ -1440,11 +1393,9 @@ extern "C" ctl_status ctl_fitness_device(const uint32_t* d_samples, uint32_t ns,
         set_error("ctl_fitness_device: invalid argument");
         return CTL_ERR_ARG;
     }
-    const uint32_t nsets = (uint32_t)(((uint64_t)threads * blocks) / p_rep);
-    dev::fitness_kernel<<<(nsets + 127) / 128, 128, 0, static_cast<cudaStream_t>(stream)>>>(
-        d_samples, d_target, d_experiment, d_fitness, threads, nsets, p_rep, ns, s_out, experiments, repetitions);
-    CTL_CUDA(cudaGetLastError());
-    return CTL_OK;
+    return launch_fitness({d_samples, nullptr, d_target, d_experiment, d_fitness, threads,
+                           (uint32_t)(((uint64_t)threads * blocks) / p_rep), p_rep, ns, s_out, experiments, repetitions},
+                          static_cast<cudaStream_t>(stream));
 }
 
 extern "C" ctl_status ctl_fitness(ctl_model* m, const ctl_target* t, const ctl_run_cfg* cfg,
@@ -1470,12 +1421,13 @@ extern "C" ctl_status ctl_fitness(ctl_model* m, const ctl_target* t, const ctl_r
     if (e == cudaSuccess && bt) e = cudaMemcpyAsync(dt, t->series.data(), bt, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(dw, t->thread2experiment.data(), bw, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(df, 0, (size_t)N * 8, s);
+    ctl_status st = CTL_OK;
     if (e == cudaSuccess && nsets) {
-        dev::fitness_kernel<<<(nsets + 127) / 128, 128, 0, s>>>(
-            static_cast<uint32_t*>(ds), static_cast<uint32_t*>(dt), static_cast<uint8_t*>(dw),
-            static_cast<double*>(df), t->threads, nsets, t->p_rep, (uint32_t)h.ns, (uint32_t)h.s_out,
-            t->experiments, t->repetitions);
-        e = cudaGetLastError();
+        st = launch_fitness({static_cast<uint32_t*>(ds), nullptr, static_cast<uint32_t*>(dt), static_cast<uint8_t*>(dw),
+                             static_cast<double*>(df), t->threads, nsets, t->p_rep, (uint32_t)h.ns, (uint32_t)h.s_out,
+                             t->experiments, t->repetitions},
+                            s);
+        if (st != CTL_OK) e = cudaErrorLaunchFailure;
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(fitness, df, (size_t)N * 8, cudaMemcpyDeviceToHost, s);
     if (ds) cudaFreeAsync(ds, s);
@@ -1484,6 +1436,7 @@ extern "C" ctl_status ctl_fitness(ctl_model* m, const ctl_target* t, const ctl_r
     if (df) cudaFreeAsync(df, s);
     cudaError_t e2 = cudaStreamSynchronize(s);
     cudaStreamDestroy(s);
+    if (st != CTL_OK) return st;
     if (e != cudaSuccess) return cuda_fail(e, "ctl_fitness");
     if (e2 != cudaSuccess) return cuda_fail(e2, "ctl_fitness (kernel)");
     return CTL_OK;
@@ -1534,12 +1487,10 @@ extern "C" ctl_status ctl_fitness_sums_device(const uint64_t* d_sums, uint32_t n
         set_error("ctl_fitness_sums_device: invalid argument");
         return CTL_ERR_ARG;
     }
-    const uint32_t nsets = (uint32_t)(((uint64_t)threads * blocks) / p_rep);
-    dev::fitness_sums_kernel<<<(nsets + 127) / 128, 128, 0, static_cast<cudaStream_t>(stream)>>>(
-        reinterpret_cast<const unsigned long long*>(d_sums), d_target, d_experiment, d_fitness, nsets, p_rep, ns,
-        s_out, experiments, repetitions);
-    CTL_CUDA(cudaGetLastError());
-    return CTL_OK;
+    return launch_fitness({nullptr, reinterpret_cast<const unsigned long long*>(d_sums), d_target, d_experiment, d_fitness,
+                           threads, (uint32_t)(((uint64_t)threads * blocks) / p_rep), p_rep, ns, s_out, experiments,
+                           repetitions},
+                          static_cast<cudaStream_t>(stream));
 }
 
 extern "C" ctl_status ctl_fitness_run(ctl_model* m, const ctl_target* t, const ctl_run_cfg* cfg, const int32_t* X0,
@@ -1596,11 +1547,11 @@ extern "C" ctl_status ctl_fitness_run(ctl_model* m, const ctl_target* t, const c
         if (st != CTL_OK) e = cudaErrorLaunchFailure;
     }
     if (e == cudaSuccess && nsets) {
-        dev::fitness_sums_kernel<<<(nsets + 127) / 128, 128, 0, s>>>(
-            static_cast<unsigned long long*>(dsum), static_cast<uint32_t*>(dt), static_cast<uint8_t*>(dw),
-            static_cast<double*>(df), nsets, t->p_rep, (uint32_t)h.ns, (uint32_t)h.s_out, t->experiments,
-            t->repetitions);
-        e = cudaGetLastError();
+        st = launch_fitness({nullptr, static_cast<unsigned long long*>(dsum), static_cast<uint32_t*>(dt),
+                             static_cast<uint8_t*>(dw), static_cast<double*>(df), t->threads, nsets, t->p_rep,
+                             (uint32_t)h.ns, (uint32_t)h.s_out, t->experiments, t->repetitions},
+                            s);
+        if (st != CTL_OK) e = cudaErrorLaunchFailure;
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(fitness, df, (size_t)N * 8, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(info, dinf, bi, cudaMemcpyDeviceToHost, s);
