@@ -91,8 +91,9 @@ struct Run {
 // Random numbers and elementary functions (bitwise identical to the oracle)
 // ---------------------------------------------------------------------------
 
+template <int UNROLL = 10>
 __device__ __forceinline__ uint4 philox10(uint4 c, uint32_t k0, uint32_t k1) {
-#pragma unroll
+#pragma unroll UNROLL
     for (int i = 0; i < 10; i++) {
         uint32_t hi0 = __umulhi(0xD2511F53u, c.x), lo0 = 0xD2511F53u * c.x;
         uint32_t hi1 = __umulhi(0xCD9E8D57u, c.z), lo1 = 0xCD9E8D57u * c.z;
@@ -106,6 +107,13 @@ __device__ __forceinline__ uint4 philox10(uint4 c, uint32_t k0, uint32_t k1) {
 __device__ __forceinline__ uint4 draw(uint64_t seed, uint32_t blk, uint32_t tag, uint32_t step,
                                       uint32_t sim) {
     return philox10(make_uint4(blk, tag, step, sim), (uint32_t)seed, (uint32_t)(seed >> 32));
+}
+
+// The same block from half the code, for callers whose loops the instruction
+// cache would otherwise not hold (the shared-memory sweep's leap: 64 x 128
+// network on one B200, 253 -> 242 ms).
+__device__ __forceinline__ uint4 draw_small(uint64_t seed, uint32_t blk, uint32_t tag, uint32_t step, uint32_t sim) {
+    return philox10<5>(make_uint4(blk, tag, step, sim), (uint32_t)seed, (uint32_t)(seed >> 32));
 }
 
 __device__ __forceinline__ double u32d(uint32_t w) { return ((double)w + 0.5) * 0x1p-32; }
@@ -241,25 +249,56 @@ static __constant__ double c_recip[64] = {
     0x1.1f7047dc11f70p-6, 0x1.1a7b9611a7b96p-6, 0x1.15b1e5f75270dp-6, 0x1.1111111111111p-6,
     0x1.0c9714fbcda3bp-6, 0x1.0842108421084p-6, 0x1.0410410410410p-6, 0x1.0000000000000p-6};
 
+// exp(-lam) for 0 <= lam < 10: dexp's reduction, polynomial and scaling
+// without its tests for arguments out of range.
+__device__ __forceinline__ double dexp_neg10(double lam) {
+    const double x = -lam;
+    double k = rint(x * 0x1.71547652b82fep+0);
+    double r = fma(-k, CTL_LN2_HI, x);
+    r = fma(-k, CTL_LN2_LO, r);
+    double p = 0x1.93974a8c07c9dp-37;
+    p = fma(p, r, 0x1.6124613a86d09p-33);
+    p = fma(p, r, 0x1.1eed8eff8d898p-29);
+    p = fma(p, r, 0x1.ae64567f544e4p-26);
+    p = fma(p, r, 0x1.27e4fb7789f5cp-22);
+    p = fma(p, r, 0x1.71de3a556c734p-19);
+    p = fma(p, r, 0x1.a01a01a01a01ap-16);
+    p = fma(p, r, 0x1.a01a01a01a01ap-13);
+    p = fma(p, r, 0x1.6c16c16c16c17p-10);
+    p = fma(p, r, 0x1.1111111111111p-7);
+    p = fma(p, r, 0x1.5555555555555p-5);
+    p = fma(p, r, 0x1.5555555555555p-3);
+    p = fma(p, r, 0.5);
+    p = fma(p, r, 1.0);
+    p = fma(p, r, 1.0);
+    return p * __longlong_as_double((long long)((uint64_t)((int)k + 1023) << 52));
+}
+
 // Poisson(lam) given the reaction's primary uniform pair (wa, wb).
 // lam < 10: sequential inversion, p_k = p_{k-1} lam (1/k) with tabulated
-// reciprocals.  lam >= 10: Hormann's PTRS (1993); extra
-// trials read blocks 1 + 2j + odd of the same (tag, step, sim) stream.
-static __device__ uint32_t poisson(double lam, uint32_t wa, uint32_t wb, uint64_t seed, uint32_t tag,
-                            uint32_t step, uint32_t sim, uint32_t odd) {
+// reciprocals.  Four terms per trip: the cumulative sum never falls, so the
+// count is the number of partial sums below u.
+__device__ __forceinline__ uint32_t poisson_inversion(double lam, uint32_t wa) {
     if (!(lam > 0.0)) return 0u;
-    if (lam < 10.0) {
-        double u = u32d(wa);
-        double p = dexp(-lam);
-        double F = p;
-        uint32_t k = 0;
-        while (u > F && k < 64u) {
-            k = k + 1u;
-            p = (p * lam) * c_recip[k - 1u];
+    const double u = u32d(wa);
+    double p = dexp_neg10(lam);
+    double F = p;
+    uint32_t k = 0;
+    for (uint32_t i = 0; i < 64u && u > F; i += 4u) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            k += u > F ? 1u : 0u;
+            p = (p * lam) * c_recip[i + j];
             F = F + p;
         }
-        return k;
     }
+    return k;
+}
+
+// lam >= 10: Hormann's PTRS (1993); extra trials read blocks 1 + 2j + odd of
+// the same (tag, step, sim) stream.
+__device__ __forceinline__ uint32_t poisson_ptrs(double lam, uint32_t wa, uint32_t wb, uint64_t seed, uint32_t tag,
+                                                 uint32_t step, uint32_t sim, uint32_t odd) {
     double slam = sqrt(lam);
     double b = 0.931 + 2.53 * slam;
     double a = -0.059 + 0.02483 * b;
@@ -272,7 +311,7 @@ static __device__ uint32_t poisson(double lam, uint32_t wa, uint32_t wb, uint64_
     for (uint32_t t = 0; t < PTRS_MAX_TRIALS; t++) {
         if (t > 0) {
             uint32_t j = (t - 1) >> 1;
-            if (((t - 1) & 1u) == 0u) w = draw(seed, 1u + 2u * j + odd, tag, step, sim);
+            if (((t - 1) & 1u) == 0u) w = draw_small(seed, 1u + 2u * j + odd, tag, step, sim);
             wa = ((t - 1) & 1u) ? w.z : w.x;
             wb = ((t - 1) & 1u) ? w.w : w.y;
         }
@@ -294,6 +333,27 @@ static __device__ uint32_t poisson(double lam, uint32_t wa, uint32_t wb, uint64_
     return clamp_k(floor(lam));
 }
 
+// The first trial of poisson_ptrs as far as its squeeze: true with the count
+// when that accepts.
+__device__ __forceinline__ bool poisson_ptrs_quick(double lam, uint32_t wa, uint32_t wb, uint32_t& k_out) {
+    double slam = sqrt(lam);
+    double b = 0.931 + 2.53 * slam;
+    double a = -0.059 + 0.02483 * b;
+    double vr = 0.9277 - 3.6224 / (b - 2.0);
+    double U = u32d(wa) - 0.5;
+    double V = u32d(wb);
+    double us = 0.5 - fabs(U);
+    double k = floor((2.0 * a / us + b) * U + lam + 0.43);
+    k_out = clamp_k(k);
+    return us >= 0.07 && V <= vr;
+}
+
+static __device__ uint32_t poisson(double lam, uint32_t wa, uint32_t wb, uint64_t seed, uint32_t tag,
+                            uint32_t step, uint32_t sim, uint32_t odd) {
+    if (lam < 10.0 || !(lam > 0.0)) return poisson_inversion(lam, wa);
+    return poisson_ptrs(lam, wa, wb, seed, tag, step, sim, odd);
+}
+
 // Cao's g_i (tau.cu:1741-1789) in FP32.
 __device__ __forceinline__ float gfun(uint32_t hor, uint32_t hort, int32_t x) {
     float xf = (float)x;
@@ -309,11 +369,13 @@ __device__ __forceinline__ float gfun(uint32_t hor, uint32_t hort, int32_t x) {
 }
 
 // One binary level: left unless the target lies beyond a positive left
-// weight and the right weight is positive.
+// weight and the right weight is positive.  Weights are >= 0 and the target is
+// positive and stays so (a uniform above 0 times a positive sum, less a left
+// weight it exceeds), so "beyond" is x > L also where L is 0.
 __device__ __forceinline__ bool go_right(double& x, double L, double R) {
-    if ((x <= L && L > 0.0) || R == 0.0) return false;
-    x = x - L;
-    return true;
+    const bool right = (x > L) & (R != 0.0);
+    if (right) x = x - L;
+    return right;
 }
 
 

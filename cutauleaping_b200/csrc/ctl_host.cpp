@@ -101,9 +101,11 @@ ctl_status build_tables(int S, int R, const int32_t* left, const int32_t* right,
             if (left[(size_t)r * S + s] > 0) t.reac_ent.push_back(pack((uint32_t)s, left[(size_t)r * S + s]));
         t.reac_off.push_back((uint32_t)t.reac_ent.size());
     }
-    // Packed reactant descriptors: the common case of at most two reactant
-    // entries with coefficients 1 or 2 needs one table load per propensity.
-    t.reac_desc.assign((size_t)2 * R, 0u);
+    // Packed reactant descriptors (species * 4 + coefficient): the common case
+    // of at most two reactant entries with coefficients 1 or 2 needs one table
+    // load per propensity.  A missing entry is the dummy species S with
+    // coefficient 0; 0xffffffff: the general list.
+    t.reac_desc.assign((size_t)2 * R, (uint32_t)S * 4u);
     for (int r = 0; r < R; r++) {
         const uint32_t e0 = t.reac_off[r], e1 = t.reac_off[r + 1];
         bool simple = e1 - e0 <= 2;
@@ -112,7 +114,8 @@ ctl_status build_tables(int S, int R, const int32_t* left, const int32_t* right,
             t.reac_desc[2 * r] = 0xffffffffu;
             continue;
         }
-        for (uint32_t e = e0; e < e1; e++) t.reac_desc[2 * r + (e - e0)] = t.reac_ent[e];
+        for (uint32_t e = e0; e < e1; e++)
+            t.reac_desc[2 * r + (e - e0)] = (t.reac_ent[e] >> 8) * 4u + (t.reac_ent[e] & 0xffu);
     }
     // V species-major = RAV (tau.cu:314-326); F species-major and reaction-major
     t.vs_off.push_back(0);
@@ -147,6 +150,13 @@ ctl_status build_tables(int S, int R, const int32_t* left, const int32_t* right,
         t.dep_ent.insert(t.dep_ent.end(), tmp.begin(), tmp.end());
         t.dep_off.push_back((uint32_t)t.dep_ent.size());
     }
+    // What a firing of r reads, in two loads: where its row of F and its
+    // dependents lie, then each dependent with its descriptors.
+    for (int r = 0; r < R; r++)
+        for (uint32_t v : {t.fr_off[r], t.fr_off[r + 1] - t.fr_off[r], t.dep_off[r], t.dep_off[r + 1] - t.dep_off[r]})
+            t.fire.push_back(v);
+    for (uint32_t r : t.dep_ent)
+        for (uint32_t v : {r, t.reac_desc[2 * r], t.reac_desc[2 * r + 1], r ^ ((r >> 3) & 12u)}) t.dep.push_back(v);
     // HOR / HORtype exactly as tau.cu:402-432 (order-dependent hortype).
     t.hor.assign((size_t)S, 0);
     t.hort.assign((size_t)S, 0);
@@ -162,6 +172,23 @@ ctl_status build_tables(int S, int R, const int32_t* left, const int32_t* right,
             if (l > 0 && order[r] > t.hor[s]) { t.hor[s] = order[r]; t.hort[s] = (uint8_t)l; }
             if (t.hort[s] < l) t.hort[s] = (uint8_t)l;
         }
+    // Species by their entries, most first: the order in which the device's
+    // lanes take them.
+    auto by_entries = [&](const std::vector<uint32_t>& off, std::vector<uint32_t>& sp) {
+        std::vector<uint32_t> order_s((size_t)S);
+        for (int s = 0; s < S; s++) order_s[s] = (uint32_t)s;
+        std::stable_sort(order_s.begin(), order_s.end(),
+                         [&](uint32_t a, uint32_t b) { return off[a + 1] - off[a] > off[b + 1] - off[b]; });
+        for (uint32_t s : order_s)
+            for (uint32_t v : {s, off[s], off[s + 1] - off[s], (uint32_t)t.hor[s] | (uint32_t)t.hort[s] << 8})
+                sp.push_back(v);
+    };
+    by_entries(t.vs_off, t.vs_sp);
+    by_entries(t.fs_off, t.fs_sp);
+    for (int r = 0; r < R; r++) {
+        t.general = t.general || t.reac_desc[2 * r] == 0xffffffffu;
+        t.changes = std::max(t.changes, (int)(t.fr_off[r + 1] - t.fr_off[r]));
+    }
     return CTL_OK;
 }
 

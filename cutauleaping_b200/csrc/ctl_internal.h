@@ -21,12 +21,20 @@ inline uint32_t pack(uint32_t idx, int coef) { return (idx << 8) | (uint32_t)(ui
 struct HostTables {
     int S = 0, R = 0, P = 2, logP = 1, ns = 0, s_out = 0;
     std::vector<uint32_t> reac_off, reac_ent;  // reactants (left > 0), r-major: s<<8|st
-    std::vector<uint32_t> reac_desc;           // [2R]: up to two reactant entries (s<<8|st, 0 = none);
+    std::vector<uint32_t> reac_desc;           // [2R]: two reactant entries, species * 4 + coefficient
+                                               // (species S, coefficient 0 = none);
                                                // 0xffffffff in slot 0 = use the general list
     std::vector<uint32_t> vs_off, vs_ent;      // V = right-left, species-major: r<<8|v
     std::vector<uint32_t> fs_off, fs_ent;      // F (feed-masked V), species-major: r<<8|f
     std::vector<uint32_t> fr_off, fr_ent;      // F, reaction-major: s<<8|f
     std::vector<uint32_t> dep_off, dep_ent;    // reactions whose propensity a firing changes
+    std::vector<uint32_t> fire;                // [4R]: first entry and entries of fr, first and number of dep
+    std::vector<uint32_t> dep;                 // [4 nnz_dep]: dependent reaction, its two descriptors,
+                                               // the place of its leaf (dev::leaf_pos)
+    std::vector<uint32_t> vs_sp, fs_sp;        // [4S]: species by entries of vs / fs, most first: species,
+                                               // first entry, entries, HOR | HORtype << 8
+    bool general = false;                      // some reaction needs the general reactant list
+    int changes = 0;                           // most species a reaction changes
     std::vector<uint8_t> hor, hort;            // Cao HOR / HORtype (tau.cu:402-432)
     std::vector<double> tvec;                  // sample instants
     std::vector<uint32_t> cs;                  // sampled species
@@ -38,21 +46,11 @@ struct DeviceCopy {
     void* buf = nullptr;         // all tables, one allocation
     size_t bytes = 0;
     uint32_t* ctrl = nullptr;    // [0] = work-queue ticket, [1..] spare
-    size_t off_reac_off = 0, off_reac_ent = 0, off_vs_off = 0, off_vs_ent = 0;
-    size_t off_fs_off = 0, off_fs_ent = 0, off_fr_off = 0, off_fr_ent = 0;
-    size_t off_dep_off = 0, off_dep_ent = 0, off_hor = 0, off_hort = 0, off_tvec = 0, off_cs = 0;
+    size_t off_reac_off = 0, off_reac_ent = 0, off_vs_sp = 0, off_vs_ent = 0;
+    size_t off_fs_sp = 0, off_fs_ent = 0, off_fr_ent = 0, off_fire = 0;
+    size_t off_dep = 0, off_tvec = 0, off_cs = 0;
     size_t off_reac_desc = 0;
 };
-
-// Shifts of the stored levels of the propensity sum tree over P = 2^logP
-// leaves: 3, 6, 9, ... below logP, then logP (the root).  Stored level li
-// holds the nodes that cover 2^shift leaves.
-inline int stored_level_shifts(int logP, int (&shift)[10]) {
-    int n = 0;
-    for (int l = 3; l < logP; l += 3) shift[n++] = l;
-    shift[n++] = logP;
-    return n;
-}
 
 void set_error(const std::string& msg);
 ctl_status build_tables(int S, int R, const int32_t* left, const int32_t* right,

@@ -68,16 +68,13 @@ static void table_layout(const HostTables& t, DeviceCopy& d, Place&& place) {
     d.off_reac_off = place(t.reac_off.size() * 4);
     d.off_reac_ent = place(std::max<size_t>(1, t.reac_ent.size()) * 4);
     d.off_reac_desc = place(t.reac_desc.size() * 4);
-    d.off_vs_off = place(t.vs_off.size() * 4);
+    d.off_vs_sp = place(t.vs_sp.size() * 4);
     d.off_vs_ent = place(std::max<size_t>(1, t.vs_ent.size()) * 4);
-    d.off_fs_off = place(t.fs_off.size() * 4);
+    d.off_fs_sp = place(t.fs_sp.size() * 4);
     d.off_fs_ent = place(std::max<size_t>(1, t.fs_ent.size()) * 4);
-    d.off_fr_off = place(t.fr_off.size() * 4);
     d.off_fr_ent = place(std::max<size_t>(1, t.fr_ent.size()) * 4);
-    d.off_dep_off = place(t.dep_off.size() * 4);
-    d.off_dep_ent = place(std::max<size_t>(1, t.dep_ent.size()) * 4);
-    d.off_hor = place(t.hor.size());
-    d.off_hort = place(t.hort.size());
+    d.off_fire = place(t.fire.size() * 4);
+    d.off_dep = place(std::max<size_t>(4, t.dep.size()) * 4);
     d.off_tvec = place(t.tvec.size() * 8);
     d.off_cs = place(t.cs.size() * 4);
 }
@@ -87,16 +84,13 @@ static void table_fill(const HostTables& t, const DeviceCopy& d, Put&& put) {
     put(d.off_reac_off, t.reac_off.data(), t.reac_off.size() * 4) &&
         put(d.off_reac_ent, t.reac_ent.data(), t.reac_ent.size() * 4) &&
         put(d.off_reac_desc, t.reac_desc.data(), t.reac_desc.size() * 4) &&
-        put(d.off_vs_off, t.vs_off.data(), t.vs_off.size() * 4) &&
+        put(d.off_vs_sp, t.vs_sp.data(), t.vs_sp.size() * 4) &&
         put(d.off_vs_ent, t.vs_ent.data(), t.vs_ent.size() * 4) &&
-        put(d.off_fs_off, t.fs_off.data(), t.fs_off.size() * 4) &&
+        put(d.off_fs_sp, t.fs_sp.data(), t.fs_sp.size() * 4) &&
         put(d.off_fs_ent, t.fs_ent.data(), t.fs_ent.size() * 4) &&
-        put(d.off_fr_off, t.fr_off.data(), t.fr_off.size() * 4) &&
         put(d.off_fr_ent, t.fr_ent.data(), t.fr_ent.size() * 4) &&
-        put(d.off_dep_off, t.dep_off.data(), t.dep_off.size() * 4) &&
-        put(d.off_dep_ent, t.dep_ent.data(), t.dep_ent.size() * 4) &&
-        put(d.off_hor, t.hor.data(), t.hor.size()) &&
-        put(d.off_hort, t.hort.data(), t.hort.size()) &&
+        put(d.off_fire, t.fire.data(), t.fire.size() * 4) &&
+        put(d.off_dep, t.dep.data(), t.dep.size() * 4) &&
         put(d.off_tvec, t.tvec.data(), t.tvec.size() * 8) &&
         put(d.off_cs, t.cs.data(), t.cs.size() * 4);
 }
@@ -154,31 +148,30 @@ static ctl_status ensure_device(ctl_model* m, int device, DeviceCopy*& out) {
     return CTL_OK;
 }
 
-static void tree_levels(const HostTables& t, dev::Model& dm);
+// Leaves of the device's sum tree: read four at a time.
+static int device_leaves(const HostTables& t) { return std::max(4, t.P); }
 
 static dev::Model make_dev_model(const ctl_model* m, const DeviceCopy& d, uint32_t flags) {
     const HostTables& t = m->t;
     auto P = [&](size_t o) { return static_cast<const unsigned char*>(d.buf) + o; };
     dev::Model dm;
-    dm.S = t.S; dm.R = t.R; dm.P = t.P; dm.logP = t.logP; dm.ns = t.ns; dm.s_out = t.s_out;
+    dm.S = t.S; dm.R = t.R; dm.P = device_leaves(t); dm.ns = t.ns; dm.s_out = t.s_out;
     dm.reac_off = reinterpret_cast<const uint32_t*>(P(d.off_reac_off));
     dm.reac_ent = reinterpret_cast<const uint32_t*>(P(d.off_reac_ent));
     dm.reac_desc = reinterpret_cast<const uint2*>(P(d.off_reac_desc));
     const bool q5off = (flags & dev::F_Q5_OFF) != 0;
-    dm.v_off = reinterpret_cast<const uint32_t*>(P(q5off ? d.off_fs_off : d.off_vs_off));
+    dm.general = t.general ? 1 : 0;
+    dm.changes = t.changes;
+    dm.v_sp = reinterpret_cast<const uint4*>(P(q5off ? d.off_fs_sp : d.off_vs_sp));
     dm.v_ent = reinterpret_cast<const uint32_t*>(P(q5off ? d.off_fs_ent : d.off_vs_ent));
-    dm.fs_off = reinterpret_cast<const uint32_t*>(P(d.off_fs_off));
+    dm.fs_sp = reinterpret_cast<const uint4*>(P(d.off_fs_sp));
     dm.fs_ent = reinterpret_cast<const uint32_t*>(P(d.off_fs_ent));
-    dm.fr_off = reinterpret_cast<const uint32_t*>(P(d.off_fr_off));
     dm.fr_ent = reinterpret_cast<const uint32_t*>(P(d.off_fr_ent));
-    dm.dep_off = reinterpret_cast<const uint32_t*>(P(d.off_dep_off));
-    dm.dep_ent = reinterpret_cast<const uint32_t*>(P(d.off_dep_ent));
-    dm.hor = P(d.off_hor);
-    dm.hort = P(d.off_hort);
+    dm.fire = reinterpret_cast<const uint4*>(P(d.off_fire));
+    dm.dep = reinterpret_cast<const uint4*>(P(d.off_dep));
     dm.tvec = reinterpret_cast<const double*>(P(d.off_tvec));
     dm.cs = reinterpret_cast<const uint32_t*>(P(d.off_cs));
     dm.tmax = t.tmax;
-    tree_levels(t, dm);
     return dm;
 }
 
@@ -192,62 +185,27 @@ struct LaunchPlan {
     const void* spec = nullptr;  // the kernel compiled for this network, if any
 };
 
-// Stored levels of the sum tree for P = 2^k leaves: 3, 6, ... below k, then
-// k (the root).  Level li is the pairwise sum of 2^d nodes of level li-1.
-static void tree_levels(const HostTables& t, dev::Model& dm) {
-    int shift[10];
-    const int nlev = stored_level_shifts(t.logP, shift);
-    int prev = 0, base = 0;
-    for (int li = 0; li < nlev; li++) {
-        dm.lev_shift_v[li] = shift[li];
-        dm.lev_d_v[li] = shift[li] - prev;
-        dm.lev_base_v[li] = base;
-        dm.lev_count_v[li] = t.P >> shift[li];
-        base += t.P >> shift[li];
-        prev = shift[li];
-    }
-    dm.nlev = nlev;
-}
-
-static int tree_words(const HostTables& t) {
-    dev::Model dm;
-    tree_levels(t, dm);
-    return dm.lev_base_v[dm.nlev - 1] + 1;
-}
-
 // Shared-memory bytes of a block with NS slots of group size G.
 static size_t slot_layout(const HostTables& t, int G, int NS, bool uniform_c, dev::Layout& lay, bool sums = false) {
-    size_t off = 0;
+    const int P = device_leaves(t);
+    size_t slot = dev::lay_end(t.S, P);
+    lay.oc = (uint32_t)slot;
+    if (!uniform_c) slot += (size_t)P * 4;
+    lay.olast = (uint32_t)slot;
+    if (sums) slot += (size_t)t.s_out * 4;
+    slot = align16(slot);
+    if (NS > 1 && slot % 32 == 0) slot += 16;
+    lay.slot = (uint32_t)slot;
+    lay.ns = (uint32_t)NS;
+    size_t off = (size_t)NS * slot;
     auto region = [&](size_t bytes) {
         size_t o = off;
         off = align16(off + bytes);
         return (uint32_t)o;
     };
-    const int tw = tree_words(t);
-    if (G == 1) {
-        lay.len_S = (uint32_t)t.S;
-        lay.len_P = (uint32_t)t.P;
-        lay.len_C = (uint32_t)t.P;
-        lay.len_T = (uint32_t)tw;
-        lay.len_O = (uint32_t)t.s_out;
-    } else {
-        lay.len_S = (uint32_t)(t.S | 1);
-        lay.len_P = (uint32_t)(t.P + 1);
-        lay.len_C = (uint32_t)(((t.P + 3) & ~3) + 4);
-        lay.len_T = (uint32_t)(tw | 1);
-        lay.len_O = (uint32_t)(t.s_out | 1);
-    }
-    lay.off_tree = region((size_t)NS * lay.len_T * 8);
-    lay.off_state = region((size_t)NS * (4 * 8 + 9 * 4));
-    lay.off_X = region((size_t)NS * lay.len_S * 4);
-    lay.off_X1 = region((size_t)NS * lay.len_S * 4);
-    lay.off_a = region((size_t)NS * lay.len_P * 4);
-    lay.off_K = region((size_t)NS * lay.len_P * 4);
-    lay.off_c = region(uniform_c ? (size_t)t.P * 4 : (size_t)NS * lay.len_P * 4);
-    lay.off_list = region((size_t)NS * 4);
-    lay.off_crit = region((size_t)NS * lay.len_C);
-    lay.off_grp = region((size_t)NS * (16 * (G > 32 ? G / 32 : 1) + 16));  // multi-warp group scratch
-    lay.off_last = region(sums ? (size_t)NS * lay.len_O * 4 : 0);         // fitness mode only
+    lay.off_state = region((size_t)NS * dev::STATE_BYTES);
+    lay.off_c = region(uniform_c ? (size_t)P * 4 : 0);
+    lay.off_grp = region(G > 32 ? (size_t)NS * (24 * (G / 32) + 16) : 0);  // dev::Grp<G>::SCRATCH
     return off;
 }
 
@@ -266,15 +224,15 @@ static const void* kernel_for(int G, int minb) {
     return nullptr;
 }
 
-// Lanes per simulation when the caller does not choose: about 16
-// reactions per lane up to one warp (measured best for 64 x 128: G = 8;
-// tiny networks: 1), about 8 per lane beyond (512 x 1024: G = 128, 1.8x
-// the throughput of G = 32).
+// Lanes per simulation when the caller does not choose: 16 reactions per
+// lane, so that a lane's leaves are four 16-byte loads and its part of the
+// sum tree fits its registers.  One B200, milliseconds per sweep: 64 x 128
+// network (65,536 simulations to t 2) 398 with 8 lanes, 458 with 4, 1,028
+// with 16; 32 x 64 (16,384, per-simulation rates) 104 with 4, 155 with 8;
+// 512 x 1024 (4,736 to t 0.05) 486 with 64, 514 with 32, 565 with 128.
 static int heuristic_group(const HostTables& t) {
-    const int g = t.P >= 1024 ? t.P / 8 : t.P / 16;
-    const int cap = t.P >= 1024 ? 256 : 32;
     int G = 1;
-    while (G < g && G < cap) G <<= 1;
+    while (G < t.P / 16 && G < 256) G <<= 1;
     return G;
 }
 
@@ -364,11 +322,10 @@ static ctl_status occupancy(int dev, const void* k, int threads, size_t smem, in
 // Shared-memory sweep compiled for one network (NVRTC)
 // ---------------------------------------------------------------------------
 // The kernel body of ctl_sweep_dev.cuh instantiated with the network's
-// geometry as compile-time constants: species, reactions, tree leaves, the
-// stored tree levels (shift, fan-in, offset, count), sample instants and
-// sampled species.  Loops over levels unroll and every level's offsets fold
-// into the code; the tables stay in device memory (dev::Tables, the same
-// kernel parameter as the first part of dev::Model).  On the 64 x 128
+// geometry as compile-time constants: species, reactions, tree leaves, sample
+// instants and sampled species.  Loops over a lane's leaves unroll and the
+// slots' offsets fold into the code; the tables stay in device memory
+// (dev::Tables, the same kernel parameter as the first part of dev::Model).  On the 64 x 128
 // network of the 65,536-simulation benchmark at 8 lanes per simulation this
 // takes a sweep from 1,672 to 1,232 ms on one B200, with identical bits.
 // Compiled once per process and (geometry, group size, register budget).
@@ -379,22 +336,12 @@ static ctl_status occupancy(int dev, const void* k, int threads, size_t smem, in
 static constexpr uint32_t SPEC_MIN_SIMS = 4096;
 
 static std::string sweep_spec_source(const HostTables& t, int G, int minb) {
-    dev::Model dm;
-    tree_levels(t, dm);
     std::ostringstream o;
-    o << "#define CTL_SPEC_GEOMETRY 1\n#include \"ctl_sweep_dev.cuh\"\n";
+    o << "#include \"ctl_sweep_dev.cuh\"\n";
     o << "struct ModelCT : ctl::dev::Tables {\n";
-    o << "    static constexpr int S = " << t.S << ", R = " << t.R << ", P = " << t.P << ", logP = " << t.logP
-      << ", ns = " << t.ns << ", s_out = " << t.s_out << ", nlev = " << dm.nlev << ";\n";
-    auto table = [&](const char* name, const int* v) {
-        o << "    __host__ __device__ static constexpr int " << name << "(int li) { return ";
-        for (int li = 0; li + 1 < dm.nlev; li++) o << "li == " << li << " ? " << v[li] << " : ";
-        o << v[dm.nlev - 1] << "; }\n";
-    };
-    table("lev_shift", dm.lev_shift_v);
-    table("lev_d", dm.lev_d_v);
-    table("lev_base", dm.lev_base_v);
-    table("lev_count", dm.lev_count_v);
+    o << "    static constexpr int S = " << t.S << ", R = " << t.R << ", P = " << device_leaves(t) << ", LEAVES = P, ns = " << t.ns
+      << ", s_out = " << t.s_out << ", general = " << (t.general ? 1 : 0) << ", changes = "
+      << (t.changes <= 4 ? 4 : t.changes) << ";\n";
     o << "};\n";
     o << "static_assert(sizeof(ModelCT) == sizeof(ctl::dev::Tables), \"kernel parameter layout\");\n";
     o << "extern \"C\" __global__ void __launch_bounds__(256, " << minb << ") ctl_sweep_spec("
@@ -462,13 +409,14 @@ static bool find_tuned(ctl_model* m, const ctl_run_cfg* cfg, uint32_t n, ctl_mod
     return false;
 }
 
-// SSA steps per round when neither the caller nor the tuner chose: 16, or 8
-// when the whole batch fits in one wave of resident simulations -- the
-// slowest simulation then sets the time, and its decisions wait less for the
-// block's SSA bursts (Schlogl, 4,096 simulations on one B200: 87.7k against
-// 80.2k sims/s).
-static int default_ssa_budget(bool one_wave) { return one_wave ? 8 : 16; }
-static int default_dec_budget(int G) { return G > 32 ? 2 : 1; }
+// SSA steps a warp takes with the simulations it holds before it puts them
+// back, and leap decisions likewise, when neither the caller nor the tuner
+// chose: a whole burst (64 x 128 network, 65,536 simulations on one B200: 429
+// ms with 25 steps, 408 with 50, 397 with 100), and two decisions (32 x 64 with
+// per-simulation rates: 300 ms with one, 288 with two), eight where a group
+// keeps its simulation anyway.
+static int default_ssa_budget() { return 100; }
+static int default_dec_budget(int G) { return G >= 32 ? 8 : 2; }
 
 // Launch shape of the register-resident sweep for tiny networks: one thread
 // per simulation, `warp_sims` working lanes per warp.  Library choice of
@@ -647,6 +595,11 @@ static ctl_status plan_launch(ctl_model* m, const ctl_run_cfg* cfg_in, uint32_t 
         if (device_attr(cfg->device, da0) != CTL_OK) return CTL_ERR_CUDA;
         const int gmax = std::min(t.P, 32);
         while (G < gmax && (uint64_t)n * G < (uint64_t)256 * da0.sm_count) G <<= 1;
+        // groups of several warps: half the lanes where that makes one wave of
+        // a batch that would take a little more (three blocks of 256 threads
+        // per SM hold 768 / G simulations)
+        const uint64_t cap = (uint64_t)da0.sm_count * (768 / G);
+        if (G > 32 && n > cap && n <= 2 * cap) G >>= 1;
     }
     if (G != 1 && G != 2 && G != 4 && G != 8 && G != 16 && G != 32 && G != 64 && G != 128 && G != 256) {
         set_error("group must be a power of two from 1 to 256");
@@ -664,14 +617,16 @@ static ctl_status plan_launch(ctl_model* m, const ctl_run_cfg* cfg_in, uint32_t 
     if (device_attr(dev_id, da) != CTL_OK) return CTL_ERR_CUDA;
     KernAttr ka;
     const bool uni = cfg->uniform_rates != 0;
-    // Register budget: for groups of 8 lanes or more, as many resident
-    // blocks as the slot memory of a full 256-thread block allows (2 or 3);
-    // smaller groups keep 2 (their spills cost more than the occupancy
-    // gains: Schlogl at G = 1, 62k vs 56k sims/s); 4 only when chosen or tuned.
+    // Register budget: for groups of 8 lanes or more, as many resident blocks
+    // as the slot memory of a full 256-thread block allows (2 or 3); smaller
+    // groups keep 2, and so does a batch that two blocks per SM hold (500
+    // simulations of 64 x 128 at 32 lanes on one B200: 60 ms at 3, 47 at 2,
+    // whose kernel does not spill); 4 only when chosen or tuned.
     int minb = cfg->min_blocks;
     if (minb <= 0) {
         const size_t full = slot_layout(t, G, 256 / G, uni, pl.lay, sums);
         minb = G >= 8 && 3 * (full + 1024) <= (size_t)da.smem_optin + 1024 ? 3 : 2;
+        if ((uint64_t)n * G <= (uint64_t)2 * 256 * da.sm_count) minb = 2;
     }
     // The kernel compiled for this network when asked (spec 1) or when the
     // batch is large enough to recover the compilation (spec 0), else, or
@@ -704,15 +659,30 @@ static ctl_status plan_launch(ctl_model* m, const ctl_run_cfg* cfg_in, uint32_t 
         threads -= tstep;
     }
     pl.G = G;
-    // Round budgets when neither the caller nor the tuner chose: 16 SSA steps
-    // (8 for a batch of one wave, below) and one leap decision per round (one
-    // B200, against 8 and 2: +7 % on the 64 x 128 network, +10 % on Schlogl,
-    // +12 % on the uneven batch); groups of whole warps keep two decisions
-    // (512 x 1024: 2.7 % better).
-    if (pl.dec_budget <= 0) pl.dec_budget = default_dec_budget(G);
-    pl.threads = threads;
     int bps = 0, regs = 0;
     if (ctl_status st = occupancy(dev_id, kern, threads, pl.smem, bps, regs); st != CTL_OK) return st;
+    if (const uint64_t cap = (uint64_t)bps * da.sm_count; G < 32 && pl.sched == 1 && (uint64_t)n > cap * pl.NS) {
+        // more slots than groups, as many as the resident blocks' shared
+        // memory holds (at most a quarter as many again): simulations that
+        // wait for a decision until a warp's worth has come together
+        const size_t room = ((size_t)da.smem_optin + 1024) / bps - 1024 - ((size_t)da.smem_optin - smem_max);
+        int most = std::min(pl.NS + pl.NS / 4, 32 * dev::POOL_WORDS);
+        dev::Layout lay;
+        while (most > pl.NS && slot_layout(t, G, most, uni, lay, sums) > std::min(smem_max, room)) most--;
+        // ... and no more than fill the last wave as well as the others
+        const uint64_t waves = ((uint64_t)n + cap * most - 1) / (cap * most);
+        const int ns = std::max(pl.NS, (int)(((uint64_t)n + cap * waves - 1) / (cap * waves)));
+        const size_t bytes = slot_layout(t, G, ns, uni, lay, sums);
+        int b2 = 0, r2 = 0;
+        if (ctl_status st = occupancy(dev_id, kern, threads, bytes, b2, r2); st != CTL_OK) return st;
+        if (b2 == bps) {
+            pl.lay = lay;
+            pl.smem = bytes;
+            pl.NS = ns;
+        }
+    }
+    if (pl.dec_budget <= 0) pl.dec_budget = default_dec_budget(G);
+    pl.threads = threads;
     pl.minb = minb;
     if (bps < 1) {
         set_error("sweep kernel cannot be resident with this shape");
@@ -724,7 +694,7 @@ static ctl_status plan_launch(ctl_model* m, const ctl_run_cfg* cfg_in, uint32_t 
     uint64_t need = (n + (uint64_t)pl.NS - 1) / pl.NS;
     uint64_t cap = (uint64_t)bps * da.sm_count;
     pl.blocks = (int)std::max<uint64_t>(1, std::min(need, cap));
-    if (pl.ssa_budget <= 0) pl.ssa_budget = default_ssa_budget((uint64_t)n <= (uint64_t)pl.blocks * pl.NS);
+    if (pl.ssa_budget <= 0) pl.ssa_budget = default_ssa_budget();
     return CTL_OK;
 }
 
@@ -1195,7 +1165,7 @@ extern "C" ctl_status ctl_autotune(ctl_model* m, const ctl_run_cfg* cfg, uint32_
             }
         }
         const Shape b4 = bestx;
-        for (int sb : {4, 8, 16, 32}) {                        // 5. SSA steps per round
+        for (int sb : {8, 16, 25, 50, 100}) {                  // 5. SSA steps per round
             Shape x = b4;
             x.ssa = sb;
             if (sb != b4.ssa) consider(x);
@@ -1587,7 +1557,23 @@ namespace ctl {
 // Holds the work-queue ticket (first 256 bytes) and the model tables of the
 // call in progress.  It lives in every device that loads this library, for
 // as long as the library stays loaded.
-constexpr size_t NOALLOC_BYTES = (size_t)1 << 20;
+// Models are taken by the size of their plain tables, at most 1 MiB; the
+// dependents with their descriptors, four words per dependent instead of one,
+// and the firing and species tables make the copy up to four times as large.
+constexpr size_t NOALLOC_TABLE_BYTES = (size_t)1 << 20;
+constexpr size_t NOALLOC_BYTES = 4 * NOALLOC_TABLE_BYTES;
+
+// Bytes of a model's tables with one word per dependent, each table rounded to
+// 16 bytes, after the ticket.
+static size_t plain_table_bytes(const HostTables& t) {
+    size_t n = 256;
+    for (size_t words : {t.reac_off.size(), std::max<size_t>(1, t.reac_ent.size()), t.reac_desc.size(), t.vs_off.size(),
+                         std::max<size_t>(1, t.vs_ent.size()), t.fs_off.size(), std::max<size_t>(1, t.fs_ent.size()),
+                         t.fr_off.size(), std::max<size_t>(1, t.fr_ent.size()), t.dep_off.size(),
+                         std::max<size_t>(1, t.dep_ent.size()), 2 * t.tvec.size(), t.cs.size()})
+        n += align16(words * 4);
+    return n + align16(t.hor.size()) + align16(t.hort.size());
+}
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_BYTES];
 
 static std::mutex g_noalloc_mu;
@@ -1615,9 +1601,9 @@ extern "C" ctl_status ctl_run_device_noalloc(ctl_model* m, const ctl_run_cfg* cf
         return o;
     };
     table_layout(t, d, place);
-    if (off > NOALLOC_BYTES) {
-        set_error("ctl_run_device_noalloc: the model tables need " + std::to_string(off) +
-                  " bytes, the allocation-free path holds at most " + std::to_string(NOALLOC_BYTES) +
+    if (const size_t plain = plain_table_bytes(t); plain > NOALLOC_TABLE_BYTES || off > NOALLOC_BYTES) {
+        set_error("ctl_run_device_noalloc: the model tables need " + std::to_string(plain) +
+                  " bytes, the allocation-free path holds at most " + std::to_string(NOALLOC_TABLE_BYTES) +
                   " (1 MiB); use ctl_run_device");
         return CTL_ERR_SHAPE;
     }
