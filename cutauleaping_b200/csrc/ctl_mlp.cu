@@ -884,6 +884,8 @@ __global__ void scale_kernel(double* f, uint32_t n, double s) {
 }  // namespace mlp
 }  // namespace ctl
 
+#include "ctl_train.cuh"
+
 using namespace ctl;
 
 static ctl_status mlp_cuda(cudaError_t e, const char* what) {
@@ -1112,4 +1114,167 @@ extern "C" ctl_status ctl_mlp_screen(const ctl_screen_desc* d, void* stream) {
     mlp::scale_kernel<<<(d->n_cand + 255) / 256, 256, 0, s>>>(d->fitness, d->n_cand,
                                                               1.0 / ((double)d->ns * (double)d->S));
     return mlp_cuda(cudaGetLastError(), "scale_kernel launch");
+}
+
+// ---- one training step ------------------------------------------------------------
+
+namespace {
+
+bool aligned(const void* p, size_t n) { return p && reinterpret_cast<uintptr_t>(p) % n == 0; }
+
+ctl_status check_step(const ctl_mlp_step_desc* d, const char* who) {
+    if (!d) return CTL_ERR_ARG;
+    if (d->B <= 0 || d->B % 128 || (d->out_w != 64 && d->out_w != 128)) {
+        set_error(std::string(who) + ": the batch is a positive multiple of 128 rows and out_w 64 or 128");
+        return CTL_ERR_SHAPE;
+    }
+    return CTL_OK;
+}
+
+// SM count of the current device, after raising the kernels' shared-memory
+// ceilings there once.
+ctl_status step_device(int& sms) {
+    static int known[16];
+    int dev = 0;
+    ctl_status st = mlp_cuda(cudaGetDevice(&dev), "cudaGetDevice");
+    if (st != CTL_OK) return st;
+    if (dev < 0 || dev >= 16) return CTL_ERR_ARG;
+    if (!known[dev]) {
+        const struct {
+            const void* k;
+            int bytes;
+        } ks[] = {{reinterpret_cast<const void*>(mlp::train_forward_kernel), mlp::TR_SMEM},
+                  {reinterpret_cast<const void*>(mlp::train_backward_kernel), mlp::TR_SMEM},
+                  {reinterpret_cast<const void*>(mlp::train_wgrad_kernel), mlp::WG_SMEM}};
+        for (const auto& k : ks)
+            if ((st = mlp_cuda(cudaFuncSetAttribute(k.k, cudaFuncAttributeMaxDynamicSharedMemorySize, k.bytes),
+                               "cudaFuncSetAttribute(training step)")) != CTL_OK)
+                return st;
+        int n = 0;
+        if ((st = mlp_cuda(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev), "sm count")) != CTL_OK)
+            return st;
+        known[dev] = n;
+    }
+    sms = known[dev];
+    return CTL_OK;
+}
+
+ctl_status pack_matrices(const void* const* w, const int* n, const int* k, int count, void* out, cudaStream_t s) {
+    mlp::Pack p = {};
+    size_t off = 0;
+    int most = 0;
+    for (int l = 0; l < count; l++) {
+        if (!aligned(w[l], 16)) return CTL_ERR_ARG;
+        p.w[l] = static_cast<const __nv_bfloat16*>(w[l]);
+        p.ld[l] = p.k[l] = k[l];
+        p.n[l] = n[l];
+        p.off[l] = off;
+        off += (size_t)n[l] * k[l] * 2;
+        most = std::max(most, n[l] * k[l] / 8);
+    }
+    p.out = static_cast<uint8_t*>(out);
+    mlp::train_pack_kernel<<<dim3((unsigned)((most + 255) / 256), (unsigned)count), 256, 0, s>>>(p);
+    return mlp_cuda(cudaGetLastError(), "train_pack_kernel launch");
+}
+
+}  // namespace
+
+extern "C" ctl_status ctl_mlp_forward(const ctl_mlp_step_desc* d, void* stream) {
+    ctl_status st = check_step(d, "ctl_mlp_forward");
+    if (st != CTL_OK) return st;
+    bool ok = aligned(d->X, 16) && aligned(d->wpack, 16) && aligned(d->y, 32);
+    for (int l = 0; l < mlp::TR_L; l++) ok = ok && d->bias[l] && (d->hp[l] == nullptr || aligned(d->hp[l], 16));
+    for (int l = 0; l < 4; l++) ok = ok && aligned(d->z[l], 32);
+    if (!ok) {
+        set_error("ctl_mlp_forward: a buffer is missing or not aligned");
+        return CTL_ERR_ARG;
+    }
+    int sms = 0;
+    if ((st = step_device(sms)) != CTL_OK) return st;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const int n[5] = {256, 256, 256, 256, d->out_w}, k[5] = {64, 256, 256, 256, 256};
+    if ((st = pack_matrices(d->W, n, k, 5, d->wpack, s)) != CTL_OK) return st;
+    mlp::Train p = {};
+    p.X = static_cast<const __nv_bfloat16*>(d->X);
+    p.wpack = static_cast<const uint8_t*>(d->wpack);
+    for (int l = 0; l < mlp::TR_L; l++) {
+        p.bias[l] = d->bias[l];
+        p.hp[l] = static_cast<uint8_t*>(d->hp[l]);
+    }
+    for (int l = 0; l < 4; l++) p.z[l] = d->z[l];
+    p.y = d->y;
+    p.B = d->B;
+    p.out_w = d->out_w;
+    p.err = d->err;
+    mlp::train_forward_kernel<<<d->B / 128, mlp::TR_THREADS, mlp::TR_SMEM, s>>>(p);
+    return mlp_cuda(cudaGetLastError(), "train_forward_kernel launch");
+}
+
+extern "C" ctl_status ctl_mlp_backward(const ctl_mlp_step_desc* d, void* stream) {
+    ctl_status st = check_step(d, "ctl_mlp_backward");
+    if (st != CTL_OK) return st;
+    bool ok = aligned(d->wpack, 16) && aligned(d->y, 32) && d->target && d->loss && d->S > 0 && 2 * d->S <= d->out_w;
+    for (int l = 0; l < mlp::TR_L; l++)
+        ok = ok && aligned(d->hp[l], 16) && aligned(d->dp[l], 16) && aligned(d->dW[l], 16) && d->db[l];
+    for (int l = 0; l < 4; l++) ok = ok && aligned(d->z[l], 32);
+    if (!ok) {
+        set_error("ctl_mlp_backward: a buffer is missing or not aligned, or 2 S > out_w");
+        return CTL_ERR_ARG;
+    }
+    int sms = 0;
+    if ((st = step_device(sms)) != CTL_OK) return st;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const void* w[4] = {d->WT[4], d->WT[3], d->WT[2], d->WT[1]};
+    const int n[4] = {256, 256, 256, 256}, k[4] = {d->out_w, 256, 256, 256};
+    if ((st = pack_matrices(w, n, k, 4, d->wpack, s)) != CTL_OK) return st;
+    mlp::Train p = {};
+    p.wtpack = static_cast<const uint8_t*>(d->wpack);
+    for (int l = 0; l < mlp::TR_L; l++) {
+        p.hp[l] = static_cast<uint8_t*>(d->hp[l]);
+        p.dp[l] = static_cast<uint8_t*>(d->dp[l]);
+        p.dW[l] = d->dW[l];
+        p.db[l] = d->db[l];
+    }
+    for (int l = 0; l < 4; l++) p.z[l] = d->z[l];
+    p.y = d->y;
+    p.target = d->target;
+    p.loss = d->loss;
+    p.B = d->B;
+    p.S = d->S;
+    p.out_w = d->out_w;
+    p.err = d->err;
+    mlp::train_backward_kernel<<<d->B / 128, mlp::TR_THREADS, mlp::TR_SMEM, s>>>(p);
+    if ((st = mlp_cuda(cudaGetLastError(), "train_backward_kernel launch")) != CTL_OK) return st;
+    // CTAs per layer by the layer's MMA time per 128 rows (layer 0: a quarter
+    // of the columns; the last: half the rows), one per SM in all
+    const double cost[mlp::TR_L] = {0.35, 1.0, 1.0, 1.0, 0.5};
+    const int tiles = d->B / 128;
+    mlp::WgPlan plan;
+    plan.first[0] = 0;
+    for (int l = 0; l < mlp::TR_L; l++)
+        plan.first[l + 1] = plan.first[l] + std::max(1, std::min(tiles, (int)(sms * cost[l] / 3.85)));
+    mlp::train_wgrad_kernel<<<plan.first[mlp::TR_L], mlp::TR_THREADS, mlp::WG_SMEM, s>>>(p, plan);
+    return mlp_cuda(cudaGetLastError(), "train_wgrad_kernel launch");
+}
+
+extern "C" ctl_status ctl_mlp_adam_step(const ctl_mlp_adam_desc* d, void* stream) {
+    if (!d || d->step <= 0 || (d->out_w != 64 && d->out_w != 128)) return CTL_ERR_ARG;
+    mlp::AdamAll p = {};
+    for (int l = 0; l < mlp::TR_L; l++) {
+        if (!d->w[l] || !d->g[l] || !d->m[l] || !d->v[l] || !d->b[l] || !d->gb[l] || !d->mb[l] || !d->vb[l] || !d->wb[l] ||
+            !d->wbT[l])
+            return CTL_ERR_ARG;
+        const int rows = l == 4 ? d->out_w : 256, cols = l == 0 ? 64 : 256;
+        p.w[l] = d->w[l]; p.m1[l] = d->m[l]; p.m2[l] = d->v[l]; p.g[l] = d->g[l];
+        p.w[5 + l] = d->b[l]; p.m1[5 + l] = d->mb[l]; p.m2[5 + l] = d->vb[l]; p.g[5 + l] = d->gb[l];
+        p.wb[l] = static_cast<__nv_bfloat16*>(d->wb[l]);
+        p.wbT[l] = static_cast<__nv_bfloat16*>(d->wbT[l]);
+        p.rows[l] = rows; p.cols[l] = cols;
+        p.rows[5 + l] = 1; p.cols[5 + l] = rows;
+    }
+    p.lr = d->lr; p.b1 = d->beta1; p.b2 = d->beta2; p.eps = d->eps; p.wd = d->weight_decay;
+    p.c1 = 1.0f - powf(d->beta1, (float)d->step);
+    p.c2 = 1.0f - powf(d->beta2, (float)d->step);
+    mlp::train_adam_kernel<<<dim3(64, 2 * mlp::TR_L), 256, 0, static_cast<cudaStream_t>(stream)>>>(p);
+    return mlp_cuda(cudaGetLastError(), "train_adam_kernel launch");
 }

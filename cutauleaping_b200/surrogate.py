@@ -9,9 +9,9 @@ with the plain method, which also measures the surrogate's error.
 Network: x = (8 scaled log rate constants, scaled t) -> 256 -> 256 -> 256 ->
 256 -> 2*S (per-species mean and log-variance of the standardised counts),
 SiLU, BF16 weights and activations, FP32 accumulation and master weights,
-Gaussian negative log-likelihood, Adam.  Every matrix product of training
-runs in the project's own tcgen05 kernel (ctl_mlp_gemm); the loss gradient,
-bias gradients and Adam are the project's own kernels too.  Screening runs
+Gaussian negative log-likelihood, Adam.  A training step runs in the project's
+own fused tcgen05 kernels (ctl_mlp_forward, ctl_mlp_backward) and Adam in one
+launch (ctl_mlp_adam_step); single products are ctl_mlp_gemm.  Screening runs
 the whole network and the fitness in one fused tcgen05 kernel
 (ctl_mlp_screen, `screen`).  PyTorch only provides device memory.
 """
@@ -47,6 +47,19 @@ class ScreenDesc(C.Structure):
                 ("err", C.c_void_p)]
 
 
+class StepDesc(C.Structure):
+    _fields_ = [("X", C.c_void_p), ("W", C.c_void_p * 5), ("WT", C.c_void_p * 5), ("bias", C.c_void_p * 5),
+                ("z", C.c_void_p * 4), ("y", C.c_void_p), ("hp", C.c_void_p * 5), ("dp", C.c_void_p * 5),
+                ("wpack", C.c_void_p), ("target", C.c_void_p), ("loss", C.c_void_p), ("dW", C.c_void_p * 5),
+                ("db", C.c_void_p * 5), ("B", C.c_int32), ("S", C.c_int32), ("out_w", C.c_int32), ("err", C.c_void_p)]
+
+
+class AdamDesc(C.Structure):
+    _fields_ = [(k, C.c_void_p * 5) for k in ("w", "b", "g", "gb", "m", "v", "mb", "vb", "wb", "wbT")] + \
+        [("out_w", C.c_int32), ("step", C.c_int32)] + \
+        [(k, C.c_float) for k in ("lr", "beta1", "beta2", "eps", "weight_decay")]
+
+
 def _bind():
     L = lib()
     if not getattr(L, "_mlp_bound", False):
@@ -60,6 +73,9 @@ def _bind():
         L.ctl_mlp_colsum.argtypes = [P, C.c_int32, C.c_int32, C.c_int32, P, P]
         L.ctl_mlp_adam.argtypes = [P, P, P, P, C.c_int32, C.c_int32, C.c_float, C.c_float, C.c_float,
                                    C.c_float, C.c_int32, C.c_float, P, P, P]
+        L.ctl_mlp_forward.argtypes = [C.POINTER(StepDesc), P]
+        L.ctl_mlp_backward.argtypes = [C.POINTER(StepDesc), P]
+        L.ctl_mlp_adam_step.argtypes = [C.POINTER(AdamDesc), P]
         L._mlp_bound = True
     return L
 
@@ -155,26 +171,35 @@ class MLP:
         return t
 
     def forward(self, X, keep=True):
-        """X [B][64] BF16 (B % 128 == 0) -> y [B][2S] FP32."""
+        """X [B][64] BF16 (B % 128 == 0) -> y [B][out_w] FP32, in one kernel
+        (ctl_mlp_forward).  With `keep`, what backward needs is kept too: the
+        pre-activations and the packed layer inputs."""
         torch = self.torch
+        L = _bind()
+        assert X.shape[1] == IN_PAD
+        X = X.contiguous()
         Bn = X.shape[0]
-        h = X
-        self.h = [X]
-        self.z = []
-        self.hT = []
-        for l in range(LAYERS):
-            z = self._buf(f"z{l}", (Bn, HIDDEN), torch.float32)
-            hn = self._buf(f"h{l}", (Bn, HIDDEN), torch.bfloat16)
-            hT = self._buf(f"hT{l}", (HIDDEN, Bn), torch.bfloat16) if keep else None
-            gemm(h, self.Wb[l], epilogue=EPI_BIAS_SILU, out_f32=z, out_bf=hn, out_bfT=hT,
-                 bias=self.b[l], err=self.err)
-            self.z.append(z)
-            self.h.append(hn)
-            self.hT.append(hT)
-            h = hn
+        self.z = [self._buf(f"z{l}", (Bn, HIDDEN), torch.float32) for l in range(LAYERS)]
+        self.hp = [self._buf(f"hp{l}", (Bn, IN_PAD if l == 0 else HIDDEN), torch.bfloat16)
+                   for l in range(LAYERS + 1)] if keep else None
         y = self._buf("y", (Bn, self.out_w), torch.float32)
-        gemm(h, self.Wb[LAYERS], epilogue=EPI_BIAS, out_f32=y, bias=self.b[LAYERS], err=self.err)
+        d = StepDesc()
+        d.X, d.y, d.wpack, d.err = X.data_ptr(), y.data_ptr(), self._wstage().data_ptr(), self.err.data_ptr()
+        for l in range(LAYERS + 1):
+            d.W[l], d.bias[l] = self.Wb[l].data_ptr(), self.b[l].data_ptr()
+            if l < LAYERS:
+                d.z[l] = self.z[l].data_ptr()
+            if keep:
+                d.hp[l] = self.hp[l].data_ptr()
+        d.B, d.out_w = Bn, self.out_w
+        st = L.ctl_mlp_forward(C.byref(d), _stream())
+        if st != OK:
+            raise CtlError(st, "ctl_mlp_forward")
         return y
+
+    def _wstage(self):
+        L = _bind()
+        return self._buf("wstage", (L.ctl_mlp_pack_bytes(self.out_w) // 2,), self.torch.bfloat16)
 
     def backward(self, y, target):
         """Gaussian NLL of y = [mu | log var] against target [B][S]; returns
@@ -182,51 +207,41 @@ class MLP:
         torch = self.torch
         L = _bind()
         Bn, S = target.shape
-        dy = self._buf("dy", (Bn, self.out_w), torch.bfloat16)
-        dy.zero_()
-        dyT = self._buf("dyT", (128, Bn), torch.bfloat16)
-        dyT.zero_()
-        loss = torch.zeros(1, device="cuda")
-        st = L.ctl_mlp_nll_grad(_ptr(y), y.stride(0), _ptr(target), Bn, S, _ptr(dy), dy.stride(0), _ptr(dyT), Bn,
-                                _ptr(loss), _stream())
+        y, target = y.contiguous(), target.contiguous()
+        # loss and gradients in one zeroed allocation (they are accumulated)
+        sizes = [w.numel() for w in self.W] + [b.numel() for b in self.b] + [1]
+        parts = torch.zeros(sum(sizes), device="cuda").split(sizes)
+        dW = [g.view(w.shape) for g, w in zip(parts, self.W)]
+        db, loss = list(parts[len(dW):-1]), parts[-1]
+        d = StepDesc()
+        d.y, d.target, d.loss, d.wpack = y.data_ptr(), target.data_ptr(), loss.data_ptr(), self._wstage().data_ptr()
+        for l in range(LAYERS + 1):
+            d.WT[l], d.hp[l] = self.WbT[l].data_ptr(), self.hp[l].data_ptr()
+            d.dp[l] = self._buf(f"dp{l}", (Bn, 128 if l == LAYERS else HIDDEN), torch.bfloat16).data_ptr()
+            d.dW[l], d.db[l] = dW[l].data_ptr(), db[l].data_ptr()
+            if l < LAYERS:
+                d.z[l] = self.z[l].data_ptr()
+        d.B, d.S, d.out_w, d.err = Bn, S, self.out_w, self.err.data_ptr()
+        st = L.ctl_mlp_backward(C.byref(d), _stream())
         if st != OK:
-            raise CtlError(st, "ctl_mlp_nll_grad")
-        XT = self._buf("XT", (IN_PAD, Bn), torch.bfloat16)
-        XT.copy_(self.h[0].t())
-        dW = [torch.zeros_like(w) if l < LAYERS else torch.zeros(128, HIDDEN, device="cuda")
-              for l, w in enumerate(self.W)]
-        db = [torch.zeros_like(b) for b in self.b]
-        splits = max(1, min(64, Bn // 512))
-        # output layer
-        gemm(dyT, self.hT[LAYERS - 1], epilogue=EPI_ATOMIC_F32, out_f32=dW[LAYERS], splits=splits, err=self.err)
-        L.ctl_mlp_colsum(_ptr(dy), Bn, self.out_w, self.out_w, _ptr(db[LAYERS]), _stream())
-        g = dy
-        for l in range(LAYERS - 1, -1, -1):
-            dz = self._buf(f"dz{l}", (Bn, HIDDEN), torch.bfloat16)
-            dzT = self._buf(f"dzT{l}", (HIDDEN, Bn), torch.bfloat16)
-            gemm(g, self.WbT[l + 1], epilogue=EPI_SILU_GRAD, z_in=self.z[l], out_bf=dz, out_bfT=dzT, err=self.err)
-            prevT = self.hT[l - 1] if l > 0 else XT
-            gemm(dzT, prevT, epilogue=EPI_ATOMIC_F32, out_f32=dW[l], splits=splits, err=self.err)
-            L.ctl_mlp_colsum(_ptr(dz), Bn, HIDDEN, HIDDEN, _ptr(db[l]), _stream())
-            g = dz
-        dW[LAYERS] = dW[LAYERS][: self.out_w].contiguous()
+            raise CtlError(st, "ctl_mlp_backward")
         return loss, dW, db
 
     def adam(self, dW, db, lr=1e-3, beta1=0.9, beta2=0.999, eps=1e-8, wd=0.0):
         L = _bind()
         self.step_count += 1
         self.version += 1
-        for l in range(len(self.W)):
-            rows, cols = self.W[l].shape
-            st = L.ctl_mlp_adam(_ptr(self.W[l]), _ptr(dW[l]), _ptr(self.m[l]), _ptr(self.v[l]), rows, cols,
-                                lr, beta1, beta2, eps, self.step_count, wd, _ptr(self.Wb[l]),
-                                _ptr(self.WbT[l]), _stream())
-            if st != OK:
-                raise CtlError(st, "ctl_mlp_adam")
-            st = L.ctl_mlp_adam(_ptr(self.b[l]), _ptr(db[l]), _ptr(self.mb[l]), _ptr(self.vb[l]), 1, rows,
-                                lr, beta1, beta2, eps, self.step_count, 0.0, None, None, _stream())
-            if st != OK:
-                raise CtlError(st, "ctl_mlp_adam")
+        d = AdamDesc()
+        for k, ts in (("w", self.W), ("b", self.b), ("g", dW), ("gb", db), ("m", self.m), ("v", self.v),
+                      ("mb", self.mb), ("vb", self.vb), ("wb", self.Wb), ("wbT", self.WbT)):
+            arr = getattr(d, k)
+            for l, t in enumerate(ts):
+                arr[l] = t.data_ptr()
+        d.out_w, d.step = self.out_w, self.step_count
+        d.lr, d.beta1, d.beta2, d.eps, d.weight_decay = lr, beta1, beta2, eps, wd
+        st = L.ctl_mlp_adam_step(C.byref(d), _stream())
+        if st != OK:
+            raise CtlError(st, "ctl_mlp_adam_step")
 
     def packed(self):
         """Weights in the screening kernel's streaming layout and the

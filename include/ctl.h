@@ -362,6 +362,45 @@ ctl_status ctl_mlp_adam(float* w, const float* g, float* m1, float* m2, int32_t 
                         float lr, float beta1, float beta2, float eps, int32_t step, float weight_decay,
                         void* w_bf16, void* wT_bf16, void* stream);
 
+/* One training step of the surrogate MLP (64 -> 256 x 4 -> out_w, SiLU, BF16
+ * weights and activations, FP32 accumulation; no reference counterpart) as
+ * fused kernels: the forward pass of all layers, the loss gradient with every
+ * layer's data and weight gradients, and Adam on all parameters.  All pointers
+ * are device pointers; matrices are contiguous. */
+typedef struct {
+    const void* X;          /* forward: BF16 [B][64] (16-byte aligned) */
+    const void* W[5];       /* forward: BF16 [256][64], [256][256] x 3, [out_w][256] */
+    const void* WT[5];      /* backward: their transposes (WT[0] is not read) */
+    const float* bias[5];   /* forward: [256] x 4, [out_w] */
+    float* z[4];            /* [B][256] pre-activations: written forward, read backward (32-byte aligned) */
+    float* y;               /* [B][out_w]: written forward, read backward (32-byte aligned) */
+    void* hp[5];            /* the layers' inputs in the weight gradients' order, B * 128 bytes, B * 512 x 4: written
+                               forward (where not NULL), read backward */
+    void* dp[5];            /* backward scratch: B * 512 bytes x 4, B * 256 */
+    void* wpack;            /* scratch of ctl_mlp_pack_bytes(out_w) bytes (16-byte aligned) */
+    const float* target;    /* backward: [B][S] */
+    float* loss;            /* backward: [1], the summed Gaussian NLL is added */
+    float* dW[5];           /* backward: the gradients are added (zero them first) */
+    float* db[5];
+    int32_t B, S, out_w;    /* B a multiple of 128; 2 S <= out_w, out_w 64 or 128 */
+    unsigned* err;          /* device word, bit 0 raised if a bounded wait timed out */
+} ctl_mlp_step_desc;
+ctl_status ctl_mlp_forward(const ctl_mlp_step_desc* d, void* stream);
+ctl_status ctl_mlp_backward(const ctl_mlp_step_desc* d, void* stream);
+/* ctl_mlp_adam on every weight matrix (with weight_decay) and bias vector
+ * (without) in one launch. */
+typedef struct {
+    float* w[5];
+    float* b[5];
+    const float* g[5];
+    const float* gb[5];
+    float *m[5], *v[5], *mb[5], *vb[5];
+    void *wb[5], *wbT[5];   /* the BF16 copies W and W^T, refreshed */
+    int32_t out_w, step;
+    float lr, beta1, beta2, eps, weight_decay;
+} ctl_mlp_adam_desc;
+ctl_status ctl_mlp_adam_step(const ctl_mlp_adam_desc* d, void* stream);
+
 /* Fused surrogate screening (no reference counterpart: the reference scores
  * every candidate by full simulation, kernel.cu:365-423).  For each
  * candidate parameter set, runs the trained MLP at every sample instant and
