@@ -83,6 +83,29 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsign
     return false;
 }
 
+// Warp-uniform roles.  A warp that only issues (bulk copies, MMAs) runs its loop
+// with all 32 lanes and lets one elected lane issue: the compiler then keeps
+// descriptors and addresses in uniform registers, which these instructions
+// read.  Under a lane test instead, every MMA waited for moves into uniform
+// registers: 290 cycles per MMA with its barrier work against 180 (M = 128,
+// N = 256, K = 16; 135 back to back).
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x / 32), 0); }
+__device__ __forceinline__ bool elect_one() {
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+    return e != 0;
+}
+// The whole warp waits (bounded as mbar_wait); the answer is uniform.
+__device__ __forceinline__ bool mbar_wait_u(uint64_t* bar, uint32_t parity, unsigned* err) {
+    for (uint32_t i = 0; i < WAIT_LIMIT; i++) {
+        if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+        if (i > 32) __nanosleep(64);
+    }
+    if (err && (threadIdx.x & 31) == 0) atomicOr(err, 1u);
+    return false;
+}
+__device__ __forceinline__ bool raised(int* flag) { return __any_sync(0xffffffffu, *(volatile int*)flag != 0) != 0; }
+
 __device__ __forceinline__ void fence_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
@@ -494,22 +517,33 @@ __global__ void adam_kernel(float* __restrict__ w, const float* __restrict__ g, 
 //
 // Screening scores candidates by the surrogate's ensemble mean: rows are
 // (candidate, sample instant) pairs, row = cand * ns + ti.  One persistent
-// CTA per SM works on two 128-row tiles at a time and keeps their
-// activations in shared memory for all five layers, so HBM sees only the
-// candidates' parameters and one fitness word per candidate:
-//   * warps 0-7 / 8-15 (epilogue of tile 0 / 1): build the layer-0 input
-//     rows, then per layer read the tile's TMEM accumulator (warp w owns rows
-//     32(w%4).. and column half (w/4)%2), add bias, SiLU, round to BF16 and
-//     write the next layer's A operand in place; after the last layer they
-//     accumulate sum_s |target - mean| / target per row and reduce rows to
-//     candidates in shared memory;
+// CTA per SM has two 128-row tiles under way, half a layer apart: while the
+// tensor cores run one tile's layer, the other tile's warps turn its last
+// accumulator into its next operand.  A tile's activations stay in shared
+// memory for all five layers, so HBM sees only the candidates' parameters and
+// one fitness word per candidate:
+//   * warps 0-7 / 8-15 (tile 0 / 1): build the layer-0 input rows, then per
+//     layer read the tile's TMEM accumulator (warp w owns rows 32(w%4).. and
+//     column half (w/4)%2), add bias, SiLU, round to BF16 and write the next
+//     layer's A operand in place; after the last layer sum_s |target - mean|
+//     / target per row, summed over a warp's rows of one candidate and added
+//     to its FP64 fitness;
 //   * warp 16 (producer): streams the packed weights, 32 K-columns per stage,
-//     5 stages, with bulk asynchronous copies completing on mbarriers; it
-//     runs ahead into the next layer while the epilogue works;
+//     5 stages, with bulk asynchronous copies completing on mbarriers, once
+//     per tile and layer;
 //   * warp 17 (MMA): one thread issues tcgen05.mma (M = 128, N = layer width,
-//     K = 16) for both tiles from every weight stage, so each weight byte
-//     read from L2 serves 256 rows.
-// TMEM: 512 columns, 256 per tile.
+//     K = 16), the two tiles' layers in turn.
+// TMEM: 512 columns, 256 per tile.  Bounds per tile and SM: 8,192 cycles of
+// MUFU tanh (16 per cycle), 7,200 of MMAs, 12,000 of shared-memory traffic
+// (operands 720 KB, weights 458 KB, activations and biases 400 KB).  Both tiles
+// in one step, waiting for each other's epilogues, took 34,500 cycles per tile:
+// 4,600 per layer of MMAs, 5,400 of epilogue, 1,000 of hand-over, 17,000 in the
+// final sums (32 lanes of a warp on one shared-memory word) and 6,000 in the
+// inputs.  Now 18,600: a tile's layer is 2,600 cycles of MMAs (issue: 160 per
+// MMA), 600 until the epilogue sees them, 3,600 of epilogue and 400 until the
+// next MMA; what bounds it is that chain, with two tiles in TMEM to overlap.
+// 100,000 candidates x 50 instants on one B200: 4,990 us before, 2,814 now (28
+// and 49 % of the measured BF16 rate).
 constexpr int SC_BK = 32, SC_STAGES = 5, SC_HID = 256, SC_LAYERS = 5;
 constexpr int SC_EPI = 512;                       // epilogue threads (16 warps, 8 per tile)
 constexpr int SC_THREADS = SC_EPI + 64;           // + producer and MMA warps
@@ -531,7 +565,8 @@ struct Screen {
     const float* target;  // [ns][S]
     const uint8_t* wpack; // packed BF16 weights (ctl_mlp_pack)
     const float* bias;    // [4*256 + out_w]
-    double* fit;          // [n_cand] sums, zeroed by the caller
+    double* fit;          // [n_cand], zeroed by the caller
+    double scale;         // 1 / (ns * S)
     unsigned* err;
 };
 
@@ -540,6 +575,12 @@ __device__ __forceinline__ int sc_n(const Screen& p, int l) { return l == SC_LAY
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+// One arrival for a warp's 32 lanes, each with its shared-memory writes fenced:
+// 512 arrivals on one barrier took longer than the MMAs they announced.
+__device__ __forceinline__ void mbar_arrive_warp(uint64_t* bar) {
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
 }
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
@@ -590,22 +631,11 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
 #pragma unroll
     for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
-// Named barrier 1 over the 512 epilogue threads, and the same barrier as a
-// vote: true when every epilogue thread passes true.  Barrier 2 + tile
-// covers one tile's 256 epilogue threads.
-__device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
-__device__ __forceinline__ void tile_sync(uint32_t e) { asm volatile("bar.sync %0, 256;" ::"r"(2u + e) : "memory"); }
-__device__ __forceinline__ bool epi_all(bool v) {
-    uint32_t r;
-    asm volatile(
-        "{\n\t.reg .pred a, b;\n\t"
-        "setp.ne.u32 a, %1, 0;\n\t"
-        "bar.red.and.pred b, 1, 512, a;\n\t"
-        "selp.u32 %0, 1, 0, b;\n\t}"
-        : "=r"(r)
-        : "r"((uint32_t)v)
-        : "memory");
-    return r != 0;
+// One lane waits for its warp.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, unsigned* err) {
+    bool ok = true;
+    if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, err);
+    return __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
 }
 
 // Byte offset of (row, k) in a K-major no-swizzle tile with `rows` rows.
@@ -614,34 +644,47 @@ __device__ __forceinline__ uint32_t canon(int row, int k, int rows) {
 }
 
 
+// A tile row's candidate, instant and first eight parameters, loaded while the
+// tile before it is still in its last layer.
+struct ScRow {
+    uint32_t cand, ti;
+    bool live;
+    float t, th[8];
+};
+__device__ __forceinline__ void sc_load_row(const Screen& p, uint32_t row, int h, ScRow& x) {
+    x.live = row < p.n_rows;
+    x.cand = x.live ? row / p.ns : 0u;
+    x.ti = x.live ? row - x.cand * p.ns : 0u;
+    x.t = p.tvec[x.ti];
+    const float* th = p.theta + (size_t)x.cand * p.n_par;
+#pragma unroll
+    for (int q = 0; q < 8; q++) x.th[q] = h == 0 && q < p.n_par ? th[q] : 0.0f;
+}
+
 // Layer-0 input columns [32 h, 32 h + 32) of row r of the tile: scaled log
 // parameters in [-1, 1], scaled time, zeros (the same FP32 operations as
-// surrogate.make_inputs).
-__device__ void sc_build_input(const Screen& p, uint8_t* A, int r, int h, uint32_t row) {
-    float x[32];
-    const int c0 = 32 * h;
-    const bool live = row < p.n_rows;
-    const uint32_t cand = live ? row / p.ns : 0u, ti = live ? row % p.ns : 0u;
-#pragma unroll
-    for (int q = 0; q < 32; q++) {
-        const int j = c0 + q;
-        float v = 0.0f;
-        if (live && j < p.n_par) {
-            const float lo = p.log_lo[j], hi = p.log_hi[j];
-            v = (2.0f * (p.theta[(size_t)cand * p.n_par + j] - lo)) / (hi - lo) - 1.0f;
-        } else if (live && j == p.n_par) {
-            v = (2.0f * p.tvec[ti]) / p.t_end - 1.0f;
-        }
-        x[q] = v;
-    }
+// surrogate.make_inputs).  lo, hi: the prior box in shared memory.
+__device__ __forceinline__ void sc_build_input(const Screen& p, const float* lo, const float* hi, uint8_t* A, int r, int h,
+                                               const ScRow& row) {
+    const float* th = p.theta + (size_t)row.cand * p.n_par;
+    const float tsc = (2.0f * row.t) / p.t_end - 1.0f;
 #pragma unroll
     for (int kb = 0; kb < 4; kb++) {
-        uint4 v;
-        v.x = pack_bf2(x[kb * 8 + 0], x[kb * 8 + 1]);
-        v.y = pack_bf2(x[kb * 8 + 2], x[kb * 8 + 3]);
-        v.z = pack_bf2(x[kb * 8 + 4], x[kb * 8 + 5]);
-        v.w = pack_bf2(x[kb * 8 + 6], x[kb * 8 + 7]);
-        *reinterpret_cast<uint4*>(A + canon(r, c0 + kb * 8, 128)) = v;
+        const int c = 32 * h + kb * 8;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (c <= p.n_par && row.live) {
+            float x[8];
+#pragma unroll
+            for (int q = 0; q < 8; q++) x[q] = kb == 0 && h == 0 ? row.th[q] : c + q < p.n_par ? th[c + q] : 0.0f;
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                const int j = c + q;
+                if (j < p.n_par) x[q] = (2.0f * (x[q] - lo[j])) / (hi[j] - lo[j]) - 1.0f;
+                else if (j == p.n_par) x[q] = tsc;
+            }
+            v = make_uint4(pack_bf2(x[0], x[1]), pack_bf2(x[2], x[3]), pack_bf2(x[4], x[5]), pack_bf2(x[6], x[7]));
+        }
+        *reinterpret_cast<uint4*>(A + canon(r, c, 128)) = v;
     }
 }
 
@@ -651,42 +694,53 @@ __device__ __forceinline__ uint32_t sc_my_tiles(const Screen& p) {
     return blockIdx.x < p.n_tiles ? (p.n_tiles - 1u - blockIdx.x) / gridDim.x + 1u : 0u;
 }
 
-__global__ void __launch_bounds__(SC_THREADS, 1) screen_kernel(Screen p) {
+__global__ void __launch_bounds__(SC_THREADS, 1) screen_kernel(const __grid_constant__ Screen p) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    __shared__ __align__(8) uint64_t full[SC_STAGES], empty[SC_STAGES], acc_full, a_ready, drain;
+    __shared__ __align__(8) uint64_t full[SC_STAGES], empty[SC_STAGES], acc_full[2], a_ready[2], drain;
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
-    __shared__ float s_acc[2][132];
     uint8_t* stage = smem + 2 * SC_A_BYTES;
     // per-CTA constants in shared memory: biases [4*256 + out_w], y_mean [S],
-    // y_std [S], and the target [ns][S] when it fits
+    // y_std [S], the prior box [2][n_par], and the target [ns][S] when it fits,
+    // in rows of odd length (neighbouring lanes read neighbouring instants)
     float* c_bias = reinterpret_cast<float*>(stage + SC_STAGES * SC_STAGE_BYTES);
     float* c_ym = c_bias + 4 * SC_HID + p.out_w;
     float* c_ys = c_ym + p.S;
-    float* c_tg = c_ys + p.S;
-    const bool tg_smem = (size_t)(4 * SC_HID + p.out_w + 2 * p.S + p.ns * p.S) * 4 <= (size_t)SC_CONST_BYTES;
+    float* c_lo = c_ys + p.S;
+    float* c_hi = c_lo + p.n_par;
+    float* c_tg = c_hi + p.n_par;
+    const uint32_t trow = (uint32_t)p.S | 1u;
+    const bool tg_smem =
+        (size_t)(4 * SC_HID + p.out_w + 2 * p.S + 2 * p.n_par) * 4 + (size_t)p.ns * trow * 4 <= (size_t)SC_CONST_BYTES;
     const float* tgt = tg_smem ? c_tg : p.target;
+    const uint32_t tstride = tg_smem ? trow : (uint32_t)p.S;
     for (int i = threadIdx.x; i < 4 * SC_HID + p.out_w; i += SC_THREADS) c_bias[i] = p.bias[i];
     for (int i = threadIdx.x; i < p.S; i += SC_THREADS) {
         c_ym[i] = p.y_mean[i];
         c_ys[i] = p.y_std[i];
     }
+    for (int i = threadIdx.x; i < p.n_par; i += SC_THREADS) {
+        c_lo[i] = p.log_lo[i];
+        c_hi[i] = p.log_hi[i];
+    }
     if (tg_smem)
-        for (int i = threadIdx.x; i < (int)(p.ns * p.S); i += SC_THREADS) c_tg[i] = p.target[i];
-    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+        for (int i = threadIdx.x; i < (int)(p.ns * p.S); i += SC_THREADS)
+            c_tg[(uint32_t)(i / p.S) * trow + i % p.S] = p.target[i];
+    const int warp = warp_index(), lane = threadIdx.x % 32;
     const uint32_t my = sc_my_tiles(p);
     if (threadIdx.x == 0) {
         for (int i = 0; i < SC_STAGES; i++) {
             mbar_init(&full[i], 1);
             mbar_init(&empty[i], 1);
         }
-        mbar_init(&acc_full, 1);
-        mbar_init(&a_ready, SC_EPI);
+        for (int i = 0; i < 2; i++) {
+            mbar_init(&acc_full[i], 1);
+            mbar_init(&a_ready[i], SC_EPI / 64);
+        }
         mbar_init(&drain, 1);
         abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    for (int i = threadIdx.x; i < 2 * 132; i += SC_THREADS) (&s_acc[0][0])[i] = 0.0f;
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                      ::"r"(smem_u32(&tmem_slot)), "r"(2 * SC_HID));
@@ -698,162 +752,165 @@ __global__ void __launch_bounds__(SC_THREADS, 1) screen_kernel(Screen p) {
     const uint32_t tmem = tmem_slot;
 
     if (warp == 16) {
-        // ---- producer: the weight stream, once per tile pair and layer ----
-        if (lane == 0) {
-            uint32_t idx = 0;
-            uint32_t issued[SC_STAGES] = {};  // copies issued per stage buffer
-            bool ok = true;
-            for (uint32_t i0 = 0; i0 < my && ok; i0 += 2) {
-                size_t off = 0;
-                for (int l = 0; l < SC_LAYERS && ok; l++) {
-                    const uint32_t bytes = (uint32_t)(sc_n(p, l) * SC_BK * 2);
-                    for (int ks = 0; ks < sc_k(l) / SC_BK; ks++, idx++) {
-                        const uint32_t sl = idx % SC_STAGES, round = idx / SC_STAGES;
-                        if (round > 0 && !mbar_wait(&empty[sl], (round - 1) & 1u, p.err)) { ok = false; break; }
-                        if (*(volatile int*)&abort_flag) { ok = false; break; }
-                        mbar_expect_tx(&full[sl], bytes);
-                        bulk_g2s(stage + sl * SC_STAGE_BYTES, p.wpack + off, bytes, &full[sl]);
-                        issued[sl]++;
-                        off += bytes;
+        // ---- producer: the weight stream, once per tile and layer ----
+        uint32_t sl = 0, par = 1u, issued = 0;  // stage, parity of its empty barrier (the first round passes), copies
+        bool ok = true;
+        for (uint32_t i0 = 0; i0 < my && ok; i0 += 2) {
+            size_t base = 0;
+            for (int l = 0; l < SC_LAYERS && ok; l++) {
+                const uint32_t bytes = (uint32_t)(sc_n(p, l) * SC_BK * 2);
+                const int ns = sc_k(l) / SC_BK;
+                for (uint32_t e = 0; e < (i0 + 1 < my ? 2u : 1u) && ok; e++) {
+                    if (raised(&abort_flag)) { ok = false; break; }
+                    for (int ks = 0; ks < ns; ks++) {
+                        if (!mbar_wait_u(&empty[sl], par, p.err)) { ok = false; break; }
+                        if (elect_one()) {
+                            mbar_expect_tx(&full[sl], bytes);
+                            bulk_g2s(stage + sl * SC_STAGE_BYTES, p.wpack + base + (size_t)ks * bytes, bytes, &full[sl]);
+                        }
+                        issued++;
+                        if (++sl == SC_STAGES) {
+                            sl = 0;
+                            par ^= 1u;
+                        }
                     }
                 }
+                base += (size_t)ns * bytes;
             }
-            if (!ok) {
-                atomicExch(&abort_flag, 1);
-                // let the copies in flight land before the CTA exits
-                for (int sl = 0; sl < SC_STAGES; sl++)
-                    if (issued[sl]) mbar_wait(&full[sl], (issued[sl] - 1) & 1u, nullptr);
-            }
+        }
+        if (!ok) {
+            if (lane == 0) atomicExch(&abort_flag, 1);
+            // let the copies in flight land before the CTA exits
+            for (uint32_t i = issued > SC_STAGES ? issued - SC_STAGES : 0u; i < issued; i++)
+                mbar_wait_u(&full[i % SC_STAGES], (i / SC_STAGES) & 1u, nullptr);
         }
     } else if (warp == 17) {
-        // ---- MMA issuer: every weight stage feeds both tiles ----
-        if (lane == 0) {
-            uint32_t idx = 0, nready = 0;
-            bool ok = true;
-            const uint32_t s0 = smem_u32(stage), a0 = smem_u32(smem), a1 = smem_u32(smem + SC_A_BYTES);
-            for (uint32_t i0 = 0; i0 < my && ok; i0 += 2) {
-                const bool two = i0 + 1 < my;
-                for (int l = 0; l < SC_LAYERS && ok; l++) {
-                    if (!mbar_wait(&a_ready, nready & 1u, p.err) || *(volatile int*)&abort_flag) { ok = false; break; }
-                    nready++;
+        // ---- MMA issuer: the tiles' layers in turn ----
+        uint32_t sl = 0, par = 0u, jobs = 0;
+        bool ok = true;
+        const uint32_t s0 = smem_u32(stage);
+        for (uint32_t i0 = 0; i0 < my && ok; i0 += 2) {
+            for (int l = 0; l < SC_LAYERS && ok; l++, jobs++) {
+                const int N = sc_n(p, l);
+                const uint32_t idesc = make_idesc(128, N);
+                const uint32_t kstep = (uint32_t)(2 * (N / 8) * 128), lbo = (uint32_t)((N / 8) * 128);
+                for (uint32_t e = 0; e < (i0 + 1 < my ? 2u : 1u); e++) {
+                    if (!mbar_wait_u(&a_ready[e], jobs & 1u, p.err) || raised(&abort_flag)) { ok = false; break; }
                     tc_fence_after();
-                    const int N = sc_n(p, l);
-                    const uint32_t idesc = make_idesc(128, N);
-                    for (int ks = 0; ks < sc_k(l) / SC_BK; ks++, idx++) {
-                        const uint32_t sl = idx % SC_STAGES, round = idx / SC_STAGES;
-                        if (!mbar_wait(&full[sl], round & 1u, p.err)) { ok = false; break; }
+                    const uint32_t a = smem_u32(smem + e * SC_A_BYTES), d = tmem + e * SC_HID;
+#pragma unroll 4
+                    for (int ks = 0; ks < sc_k(l) / SC_BK; ks++) {
+                        if (!mbar_wait_u(&full[sl], par, p.err)) { ok = false; break; }
                         tc_fence_after();
+                        const uint32_t b = s0 + sl * SC_STAGE_BYTES;
+                        if (elect_one()) {
 #pragma unroll
-                        for (int kk = 0; kk < SC_BK / 16; kk++) {
-                            const int k0 = ks * SC_BK + kk * 16;  // K offset in the activation tiles
-                            const uint32_t ka = (uint32_t)(k0 / 8) * 16u * 128u;
-                            const uint64_t db = make_desc(s0 + sl * SC_STAGE_BYTES + (uint32_t)(kk * 2 * (N / 8) * 128),
-                                                          (uint32_t)((N / 8) * 128), 128u);
-                            const uint32_t acc = (ks > 0 || kk > 0) ? 1u : 0u;
-                            mma_bf16(tmem, make_desc(a0 + ka, 16u * 128u, 128u), db, idesc, acc);
-                            if (two) mma_bf16(tmem + SC_HID, make_desc(a1 + ka, 16u * 128u, 128u), db, idesc, acc);
+                            for (int kk = 0; kk < SC_BK / 16; kk++)  // K offset in the activation tile: 32 ks + 16 kk
+                                mma_bf16(d, make_desc(a + (uint32_t)(ks * 4 + kk * 2) * 16u * 128u, 16u * 128u, 128u),
+                                         make_desc(b + (uint32_t)kk * kstep, lbo, 128u), idesc,
+                                         (ks > 0 || kk > 0) ? 1u : 0u);
+                            mma_commit(&empty[sl]);
                         }
-                        mma_commit(&empty[sl]);
+                        if (++sl == SC_STAGES) {
+                            sl = 0;
+                            par ^= 1u;
+                        }
                     }
-                    if (ok) mma_commit(&acc_full);
+                    if (!ok) break;
+                    if (elect_one()) mma_commit(&acc_full[e]);
                 }
             }
-            if (!ok) atomicExch(&abort_flag, 1);
-            mma_commit(&drain);  // every MMA this thread issued has completed once drain flips
-            mbar_wait(&drain, 0u, nullptr);
         }
+        if (!ok && lane == 0) atomicExch(&abort_flag, 1);
+        if (elect_one()) mma_commit(&drain);  // every MMA this warp issued has completed once drain flips
+        mbar_wait_u(&drain, 0u, nullptr);
     } else {
         // ---- epilogue: warps 8e..8e+7 serve tile e; warp w owns rows 32(w%4)..
         // (its TMEM lane quadrant) and column half h = (w/4)%2 ----
         const uint32_t e = (uint32_t)warp >> 3;
         const int q = warp & 3, h = (warp >> 2) & 1;
         const int r = q * 32 + lane;
-        const int et = (int)threadIdx.x - (int)e * 256;  // 0..255 within the tile's warps
         uint8_t* A = smem + e * SC_A_BYTES;
-        float* acc_c = s_acc[e];
         const uint32_t tbase = tmem + e * SC_HID + ((uint32_t)(q * 32) << 16);
         uint32_t nacc = 0;
         bool ok = true;
-        for (uint32_t i0 = 0; i0 < my && ok; i0 += 2) {
-            const bool mine = i0 + e < my;  // this pair has a tile for this warp group
-            const uint32_t t = blockIdx.x + (i0 + e) * gridDim.x;
-            const uint32_t row = t * 128u + (uint32_t)r;
-            if (mine) sc_build_input(p, A, r, h, row);
+        ScRow next;
+        if (e < my) sc_load_row(p, (blockIdx.x + e * gridDim.x) * 128u + (uint32_t)r, h, next);
+        for (uint32_t i = e; i < my && ok; i += 2) {
+            const bool live = next.live;
+            const uint32_t cand = live ? next.cand : 0xffffffffu, ti = next.ti;  // (rows past the end: no candidate's)
+            sc_build_input(p, c_lo, c_hi, A, r, h, next);
             fence_async_smem();
             tc_fence_before();
-            mbar_arrive(&a_ready);
-            for (int l = 0; l < SC_LAYERS; l++) {
-                bool got = mbar_wait(&acc_full, nacc & 1u, p.err);
-                got = epi_all(got && !*(volatile int*)&abort_flag);  // uniform over the epilogue
+            mbar_arrive_warp(&a_ready[e]);
+            for (int l = 0; l < SC_LAYERS - 1; l++) {
+                ok = mbar_wait_warp(&acc_full[e], nacc & 1u, p.err) && !__any_sync(0xffffffffu, *(volatile int*)&abort_flag);
                 nacc++;
-                if (!got) { ok = false; break; }
+                if (!ok) break;
                 tc_fence_after();
-                if (l < SC_LAYERS - 1) {
-                    if (mine) {
-                        const float* b = c_bias + l * SC_HID;
-                        const int c0 = 128 * h;
-                        uint32_t ra[32], rb[32];
-                        tmem_ld32_issue(tbase + (uint32_t)c0, ra);
+                const float* b = c_bias + l * SC_HID;
+                const int c0 = 128 * h;
+                uint32_t ra[32], rb[32];
+                tmem_ld32_issue(tbase + (uint32_t)c0, ra);
 #pragma unroll
-                        for (int j = 0; j < 4; j++) {  // four 32-column chunks, the next load in flight
-                            tmem_wait();
-                            uint32_t(&cur)[32] = (j & 1) ? rb : ra;
-                            if (j < 3) tmem_ld32_issue(tbase + (uint32_t)(c0 + 32 * (j + 1)), (j & 1) ? ra : rb);
-                            const int c = c0 + 32 * j;
-                            const float4* b4 = reinterpret_cast<const float4*>(b + c);
+                for (int j = 0; j < 4; j++) {  // four 32-column chunks, the next load in flight
+                    tmem_wait();
+                    uint32_t(&cur)[32] = (j & 1) ? rb : ra;
+                    if (j < 3) tmem_ld32_issue(tbase + (uint32_t)(c0 + 32 * (j + 1)), (j & 1) ? ra : rb);
+                    const int c = c0 + 32 * j;
+                    const float4* b4 = reinterpret_cast<const float4*>(b + c);
 #pragma unroll
-                            for (int k = 0; k < 4; k++) {  // 8 columns -> one 16-byte store
-                                const float4 ba = b4[2 * k], bb = b4[2 * k + 1];
-                                const uint32_t* u = cur + 8 * k;
-                                uint4 o;
-                                o.x = pack_bf2(silu(__uint_as_float(u[0]) + ba.x), silu(__uint_as_float(u[1]) + ba.y));
-                                o.y = pack_bf2(silu(__uint_as_float(u[2]) + ba.z), silu(__uint_as_float(u[3]) + ba.w));
-                                o.z = pack_bf2(silu(__uint_as_float(u[4]) + bb.x), silu(__uint_as_float(u[5]) + bb.y));
-                                o.w = pack_bf2(silu(__uint_as_float(u[6]) + bb.z), silu(__uint_as_float(u[7]) + bb.w));
-                                *reinterpret_cast<uint4*>(A + canon(r, c + 8 * k, 128)) = o;
-                            }
-                        }
+                    for (int k = 0; k < 4; k++) {  // 8 columns -> one 16-byte store
+                        const float4 ba = b4[2 * k], bb = b4[2 * k + 1];
+                        const uint32_t* u = cur + 8 * k;
+                        uint4 o;
+                        o.x = pack_bf2(silu(__uint_as_float(u[0]) + ba.x), silu(__uint_as_float(u[1]) + ba.y));
+                        o.y = pack_bf2(silu(__uint_as_float(u[2]) + ba.z), silu(__uint_as_float(u[3]) + ba.w));
+                        o.z = pack_bf2(silu(__uint_as_float(u[4]) + bb.x), silu(__uint_as_float(u[5]) + bb.y));
+                        o.w = pack_bf2(silu(__uint_as_float(u[6]) + bb.z), silu(__uint_as_float(u[7]) + bb.w));
+                        *reinterpret_cast<uint4*>(A + canon(r, c + 8 * k, 128)) = o;
                     }
-                    fence_async_smem();
-                    tc_fence_before();
-                    mbar_arrive(&a_ready);
-                } else {
-                    // fitness terms of this row: sum_s |target - mean| (/ target when
-                    // nonzero), 16-column chunks alternating between the column halves
-                    float acc = 0.0f;
-                    if (mine) {
-                        const float* b = c_bias + (SC_LAYERS - 1) * SC_HID;
-                        const uint32_t ti = row % p.ns;
-                        for (int c = 16 * h; c < p.S; c += 32) {
-                            float v[16];
-                            tmem_ld16(tbase + (uint32_t)c, v);
+                }
+                fence_async_smem();
+                tc_fence_before();
+                mbar_arrive_warp(&a_ready[e]);
+            }
+            if (!ok) break;
+            if (i + 2 < my) sc_load_row(p, (blockIdx.x + (i + 2) * gridDim.x) * 128u + (uint32_t)r, h, next);
+            ok = mbar_wait_warp(&acc_full[e], nacc & 1u, p.err) && !__any_sync(0xffffffffu, *(volatile int*)&abort_flag);
+            nacc++;
+            if (!ok) break;
+            tc_fence_after();
+            // fitness terms of this row: sum_s |target - mean| (/ target when
+            // nonzero), 16-column chunks alternating between the column halves
+            const float* b = c_bias + (SC_LAYERS - 1) * SC_HID;
+            const float* tr = tgt + (size_t)ti * tstride;
+            float acc = 0.0f;
+            for (int c = 16 * h; c < p.S; c += 32) {
+                float v[16];
+                tmem_ld16(tbase + (uint32_t)c, v);
 #pragma unroll
-                            for (int j = 0; j < 16; j++) {
-                                const int s_ = c + j;
-                                if (s_ < p.S && row < p.n_rows) {
-                                    const float mean = (v[j] + b[s_]) * c_ys[s_] + c_ym[s_];
-                                    const float tg = tgt[(size_t)ti * p.S + s_];
-                                    float d = fabsf(tg - mean);
-                                    if (tg != 0.0f) d = d / tg;
-                                    acc += d;
-                                }
-                            }
-                        }
+                for (int j = 0; j < 16; j++) {
+                    const int s_ = c + j;
+                    if (s_ < p.S) {
+                        const float mean = (v[j] + b[s_]) * c_ys[s_] + c_ym[s_];
+                        const float tg = tr[s_];
+                        const float d = fabsf(tg - mean), dq = d / (tg != 0.0f ? tg : 1.0f);
+                        acc += live ? dq : 0.0f;
                     }
-                    tc_fence_before();
-                    const uint32_t cand0 = (t * 128u) / p.ns;
-                    if (mine && row < p.n_rows && acc != 0.0f) atomicAdd(&acc_c[row / p.ns - cand0], acc);
-                    tile_sync(e);
-                    if (mine && t * 128u < p.n_rows) {
-                        const uint32_t last = (min(t * 128u + 127u, p.n_rows - 1u)) / p.ns;
-                        if ((uint32_t)et <= last - cand0) {
-                            atomicAdd(&p.fit[cand0 + et], (double)acc_c[et]);
-                            acc_c[et] = 0.0f;
-                        }
-                    }
-                    tile_sync(e);
                 }
             }
+            tc_fence_before();
+            // the warp's rows of one candidate are neighbouring lanes: a
+            // segmented sum leaves each candidate's share in its last lane
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const float up = __shfl_up_sync(0xffffffffu, acc, o);
+                const uint32_t cu = __shfl_up_sync(0xffffffffu, cand, o);
+                if (lane >= o && cu == cand) acc += up;
+            }
+            const uint32_t cn = __shfl_down_sync(0xffffffffu, cand, 1);
+            if (live && (lane == 31 || cn != cand)) atomicAdd(&p.fit[cand], (double)acc * p.scale);
         }
         if (!ok) atomicExch(&abort_flag, 1);
     }
@@ -874,11 +931,6 @@ __global__ void pack_kernel(const __nv_bfloat16* __restrict__ W, int N, int K, i
     const int ks = k / SC_BK, kin = k % SC_BK;
     const size_t o = (size_t)ks * N * SC_BK + canon(n, kin, N) / 2;
     out[o] = W[(size_t)n * ldw + k];
-}
-
-__global__ void scale_kernel(double* f, uint32_t n, double s) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) f[i] *= s;
 }
 
 }  // namespace mlp
@@ -1109,11 +1161,9 @@ extern "C" ctl_status ctl_mlp_screen(const ctl_screen_desc* d, void* stream) {
         sms[dev] = n;
     }
     const uint32_t grid = std::min<uint32_t>(p.n_tiles, (uint32_t)sms[dev]);  // one CTA per SM
+    p.scale = 1.0 / ((double)d->ns * (double)d->S);
     mlp::screen_kernel<<<grid, mlp::SC_THREADS, smem, s>>>(p);
-    if ((st = mlp_cuda(cudaGetLastError(), "screen_kernel launch")) != CTL_OK) return st;
-    mlp::scale_kernel<<<(d->n_cand + 255) / 256, 256, 0, s>>>(d->fitness, d->n_cand,
-                                                              1.0 / ((double)d->ns * (double)d->S));
-    return mlp_cuda(cudaGetLastError(), "scale_kernel launch");
+    return mlp_cuda(cudaGetLastError(), "screen_kernel launch");
 }
 
 // ---- one training step ------------------------------------------------------------

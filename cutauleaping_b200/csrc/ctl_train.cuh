@@ -121,7 +121,7 @@ __device__ __forceinline__ void tr_init(TrShared& sh, int warp) {
             mbar_init(&sh.empty[i], 1);
         }
         mbar_init(&sh.acc, 1);
-        mbar_init(&sh.ready, TR_EPI);
+        mbar_init(&sh.ready, TR_EPI / 32);
         mbar_init(&sh.drain, 1);
         sh.abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_forward_kernel(const __gr
             *reinterpret_cast<uint4*>(A + canon(r, (4 * h + kb) * 8, 128)) =
                 *reinterpret_cast<const uint4*>(p.X + row * IN_W + (4 * h + kb) * 8);
         fence_async_smem();
-        mbar_arrive(&sh.ready);
+        mbar_arrive_warp(&sh.ready);
         if (p.hp[0]) {
             tr_sync();
             tile_transpose(smem_u32(A), IN_W, IN_W, p.hp[0] + (size_t)blockIdx.x * 128 * IN_W * 2, nullptr, warp, lane);
@@ -283,7 +283,7 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_forward_kernel(const __gr
             if (l < TR_L - 1) {
                 fence_async_smem();
                 tc_fence_before();
-                mbar_arrive(&sh.ready);
+                mbar_arrive_warp(&sh.ready);
                 if (p.hp[l + 1]) {
                     tr_sync();
                     tile_transpose(smem_u32(A), SC_HID, SC_HID, p.hp[l + 1] + (size_t)blockIdx.x * TR_A_BYTES, nullptr,
@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_backward_kernel(const __g
             if (lane == 0 && l != 0.0f) atomicAdd(p.loss, l);
         }
         fence_async_smem();
-        mbar_arrive(&sh.ready);
+        mbar_arrive_warp(&sh.ready);
         tr_sync();
         tile_transpose(smem_u32(A), out_w, 128, p.dp[4] + (size_t)blockIdx.x * 128 * 128 * 2, p.db[4], warp, lane);
         for (int i = 0; i < 4; i++) {
@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_backward_kernel(const __g
             }
             fence_async_smem();
             tc_fence_before();
-            if (l > 0) mbar_arrive(&sh.ready);
+            if (l > 0) mbar_arrive_warp(&sh.ready);
             tr_sync();
             tile_transpose(smem_u32(A), SC_HID, SC_HID, p.dp[l] + (size_t)blockIdx.x * TR_A_BYTES, p.db[l], warp, lane);
         }

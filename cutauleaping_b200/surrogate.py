@@ -297,15 +297,18 @@ def screen(net: MLP, theta_log, tvec, target, sc: Scaling):
     tvec [ns], target [ns][S]; returns a FP64 device tensor [n]."""
     torch = net.torch
     L = _bind()
-    dev = lambda a: torch.as_tensor(np.asarray(a), dtype=torch.float32, device="cuda").contiguous()
     theta = theta_log.to(torch.float32).contiguous()
     n, n_par = theta.shape
-    tv, tg = dev(tvec), dev(target)
-    lo, hi, ym, ys = dev(sc.log_lo), dev(sc.log_hi), dev(sc.y_mean), dev(sc.y_std)
+    # the small host arrays in one copy
+    parts = [np.asarray(a, dtype=np.float32).reshape(-1)
+             for a in (tvec, target, sc.log_lo, sc.log_hi, sc.y_mean, sc.y_std)]
+    buf = torch.from_numpy(np.concatenate(parts)).cuda()
+    tv, tg, lo, hi, ym, ys = (C.c_void_p(buf.data_ptr() + 4 * o)
+                              for o in np.cumsum([0] + [p.size for p in parts[:-1]]).tolist())
     wp, bias = net.packed()
     fit = torch.empty(n, dtype=torch.float64, device="cuda")
-    d = ScreenDesc(_ptr(theta), n_par, n, _ptr(tv), tv.shape[0], float(sc.t_end), _ptr(lo), _ptr(hi), _ptr(ym),
-                   _ptr(ys), net.S, net.out_w, _ptr(tg), _ptr(wp), _ptr(bias), _ptr(fit), _ptr(net.err))
+    d = ScreenDesc(_ptr(theta), n_par, n, tv, parts[0].size, float(sc.t_end), lo, hi, ym, ys, net.S, net.out_w, tg,
+                   _ptr(wp), _ptr(bias), _ptr(fit), _ptr(net.err))
     st = L.ctl_mlp_screen(C.byref(d), _stream())
     if st != OK:
         raise CtlError(st, "ctl_mlp_screen")
