@@ -122,37 +122,106 @@ __device__ __forceinline__ double u53(uint32_t wa, uint32_t wb) {
     return ((double)m + 0.5) * 0x1p-52;
 }
 
+// Correctly rounded quotients and roots in straight-line code (Markstein
+// 1990): the approximate reciprocal is refined until it is the rounded one,
+// and the quotient corrected by its exact remainder; a root likewise from the
+// approximate reciprocal root (Goldschmidt's two products).  A general division's
+// test for special operands and the call behind it end the code that the
+// scheduler can overlap: without them an exact step of a lone Schlogl
+// simulation takes 0.29 instead of 0.50 us, and 65,537 perturbed simulations,
+// with many PTRS draws, 73 instead of 81 ms.  For operands whose reciprocal,
+// quotient and remainder stay in the normal range (the callers'), a = 0
+// included.  A divisor whose significand is all ones is the one that refines to
+// a neighbour of its rounded reciprocal; some quotients by it (a power of two
+// above it) are then the lower neighbour.
+__device__ __forceinline__ float div_near(float a, float b) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+    y = fmaf(fmaf(-b, y, 1.0f), y, y);
+    y = fmaf(fmaf(-b, y, 1.0f), y, y);
+    const float q = a * y;
+    return fmaf(fmaf(-b, q, a), y, q);
+}
+
+__device__ __forceinline__ double div_near(double a, double b) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    y = fma(fma(-b, y, 1.0), y, y);
+    y = fma(fma(-b, y, 1.0), y, y);
+    y = fma(fma(-b, y, 1.0), y, y);
+    const double q = a * y;
+    return fma(fma(-b, q, a), y, q);
+}
+
+__device__ __forceinline__ double sqrt_near(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    double g = x * y, h = 0.5 * y;
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const double r = fma(-g, h, 0.5);
+        g = fma(g, r, g);
+        h = fma(h, r, h);
+    }
+    return fma(fma(-g, g, x), h, g);
+}
+
+// Whether div_near divides by b exactly as `/` for any a that is 0 or within
+// 2^-30 .. 2^60 (num_fits: 0 or 2^-30 <= |a| < 2^30).
+__device__ __forceinline__ bool div_fits(float b) {
+    const uint32_t u = __float_as_uint(b) & 0x7fffffffu;
+    return u - 0x21800000u < 0x5d800000u - 0x21800000u && (u & 0x7fffffu) != 0x7fffffu;  // 2^-60 <= |b| < 2^60
+}
+__device__ __forceinline__ bool num_fits(float a) {
+    const uint32_t u = __float_as_uint(a) & 0x7fffffffu;
+    return u == 0u || u - 0x30800000u < 0x4e800000u - 0x30800000u;
+}
+
 #define CTL_LN2_HI 0x1.62e42fee00000p-1
 #define CTL_LN2_LO 0x1.a39ef35793c76p-33
 
-// log(x) = e ln2 + 2 atanh(s), s = (m-1)/(m+1), m in (sqrt(1/2), sqrt(2)].
+// log(x) = e ln2 + 2 atanh(s), s = (m-1)/(m+1), m in (sqrt(1/2), sqrt(2)], of
+// N positive normal numbers at once: the polynomials' steps interleave, so
+// that N logarithms take little longer than one.
+template <int N>
+__device__ __forceinline__ void dlog_of(const double (&x)[N], double (&out)[N], int eadj = 0) {
+    double ed[N], s[N], z[N], p[N];
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        const uint64_t b = (uint64_t)__double_as_longlong(x[i]);
+        int e = (int)((b >> 52) & 0x7ff) - 1023 + eadj;
+        double m = __longlong_as_double((long long)((b & 0x000fffffffffffffULL) | 0x3ff0000000000000ULL));
+        if (m > 0x1.6a09e667f3bcdp+0) { m = m * 0.5; e = e + 1; }
+        const double f = m - 1.0;
+        s[i] = div_near(f, 2.0 + f);
+        if (f == -0x1p-52) s[i] = -0x1.0000000000001p-53;  // the divisor of all ones
+        z[i] = s[i] * s[i];
+        p[i] = 0x1.8618618618618p-5;
+        ed[i] = (double)e;
+    }
+    constexpr double C[9] = {0x1.af286bca1af28p-5, 0x1.e1e1e1e1e1e1ep-5, 0x1.1111111111111p-4, 0x1.3b13b13b13b14p-4,
+                             0x1.745d1745d1746p-4, 0x1.c71c71c71c71cp-4, 0x1.2492492492492p-3, 0x1.999999999999ap-3,
+                             0x1.5555555555555p-2};
+#pragma unroll
+    for (int k = 0; k < 9; k++)
+#pragma unroll
+        for (int i = 0; i < N; i++) p[i] = fma(p[i], z[i], C[k]);
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        const double r = z[i] * p[i], two_s = s[i] + s[i];
+        out[i] = fma(ed[i], CTL_LN2_HI, two_s + fma(two_s, r, ed[i] * CTL_LN2_LO));
+    }
+}
+
 static __device__ double dlog(double x) {
     if (!(x > 0.0)) return x == 0.0 ? __longlong_as_double(0xfff0000000000000ULL)
                                      : __longlong_as_double(0x7ff8000000000000ULL);
     if (x == __longlong_as_double(0x7ff0000000000000ULL)) return x;
-    int eadj = 0;
-    if (x < 0x1p-1022) { x = x * 0x1p54; eadj = -54; }
-    uint64_t b = (uint64_t)__double_as_longlong(x);
-    int e = (int)((b >> 52) & 0x7ff) - 1023 + eadj;
-    double m = __longlong_as_double((long long)((b & 0x000fffffffffffffULL) | 0x3ff0000000000000ULL));
-    if (m > 0x1.6a09e667f3bcdp+0) { m = m * 0.5; e = e + 1; }
-    double f = m - 1.0;
-    double s = f / (2.0 + f);
-    double z = s * s;
-    double p = 0x1.8618618618618p-5;
-    p = fma(p, z, 0x1.af286bca1af28p-5);
-    p = fma(p, z, 0x1.e1e1e1e1e1e1ep-5);
-    p = fma(p, z, 0x1.1111111111111p-4);
-    p = fma(p, z, 0x1.3b13b13b13b14p-4);
-    p = fma(p, z, 0x1.745d1745d1746p-4);
-    p = fma(p, z, 0x1.c71c71c71c71cp-4);
-    p = fma(p, z, 0x1.2492492492492p-3);
-    p = fma(p, z, 0x1.999999999999ap-3);
-    p = fma(p, z, 0x1.5555555555555p-2);
-    double r = z * p;
-    double ed = (double)e;
-    double two_s = s + s;
-    return fma(ed, CTL_LN2_HI, two_s + fma(two_s, r, ed * CTL_LN2_LO));
+    const bool small = x < 0x1p-1022;
+    const double in[1] = {small ? x * 0x1p54 : x};
+    double out[1];
+    dlog_of<1>(in, out, small ? -54 : 0);
+    return out[0];
 }
 
 // exp(x): Cody-Waite reduction, degree-14 Taylor polynomial, 2^k scaling.
@@ -191,7 +260,8 @@ __device__ __forceinline__ float flog(float x) {
     float m = __uint_as_float((b & 0x007fffffu) | 0x3f800000u);
     if (m > 0x1.6a09e6p+0f) { m = m * 0.5f; e = e + 1; }
     const float f = m - 1.0f;
-    const float sv = f / (2.0f + f);
+    float sv = div_near(f, 2.0f + f);
+    sv = f == -0x1p-23f ? -0x1.000002p-24f : sv;  // the divisor of all ones
     const float z = sv * sv;
     float p = 0x1.c71c72p-4f;
     p = fmaf(p, z, 0x1.24924ap-3f);
@@ -333,25 +403,60 @@ __device__ __forceinline__ uint32_t poisson_ptrs(double lam, uint32_t wa, uint32
     return clamp_k(floor(lam));
 }
 
+// poisson_ptrs after a first trial (wa, wb) that the squeeze did not accept,
+// for the shortest chain of dependent operations: straight-line quotients, and
+// the five logarithms of the acceptance test side by side (a lone leaping
+// Schlogl simulation: 4.0 -> 3.3 us a leap, with tau_bound's).  Below a mean of 2^40 every operand, k (below 2^50) included,
+// is in their range; a larger one takes poisson_ptrs.  The shared-memory sweep,
+// whose registers are short, is faster with that (32 x 64 network: 221 against 231 ms).
+static __device__ __noinline__ uint32_t poisson_ptrs_call(double lam, uint32_t wa, uint32_t wb, uint64_t seed,
+                                                          uint32_t tag, uint32_t step, uint32_t sim, uint32_t odd) {
+    return poisson_ptrs(lam, wa, wb, seed, tag, step, sim, odd);
+}
+__device__ __forceinline__ uint32_t poisson_ptrs_wide(double lam, uint32_t wa, uint32_t wb, uint64_t seed, uint32_t tag,
+                                                      uint32_t step, uint32_t sim, uint32_t odd) {
+    if (!(lam < 0x1p40)) return poisson_ptrs_call(lam, wa, wb, seed, tag, step, sim, odd);
+    const double b = 0.931 + 2.53 * sqrt_near(lam), a = -0.059 + 0.02483 * b;
+    const double vr = 0.9277 - div_near(3.6224, b - 2.0);
+    uint4 w = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll 1
+    for (uint32_t t = 0; t < PTRS_MAX_TRIALS; t++) {
+        if (t > 0) {
+            const uint32_t j = (t - 1) >> 1;
+            if (((t - 1) & 1u) == 0u) w = draw_small(seed, 1u + 2u * j + odd, tag, step, sim);
+            wa = ((t - 1) & 1u) ? w.z : w.x;
+            wb = ((t - 1) & 1u) ? w.w : w.y;
+        }
+        const double U = u32d(wa) - 0.5, V = u32d(wb), us = 0.5 - fabs(U);
+        const double k = floor((div_near(2.0 * a, us) + b) * U + lam + 0.43);
+        if (us >= 0.07 && V <= vr) return clamp_k(k);
+        if (k < 0.0 || (us < 0.013 && V > us)) continue;
+        const double x[5] = {V, 1.1239 + div_near(1.1328, b - 3.4), div_near(a, us * us) + b, lam, k + 1.0};
+        double l[5];
+        dlog_of<5>(x, l);
+        const double ix = div_near(1.0, x[4]), ix2 = ix * ix;  // dlogfact(k)
+        const double ser = ix * (0x1.5555555555555p-4 -
+                                 ix2 * (0x1.6c16c16c16c17p-9 -
+                                        ix2 * (0x1.a01a01a01a01ap-11 - ix2 * 0x1.3813813813814p-11)));
+        const double lf = k < 16.0 ? c_logfact[(int)k] : (x[4] - 0.5) * l[4] - x[4] + 0x1.d67f1c864beb5p-1 + ser;
+        if (l[0] + l[1] - l[2] <= -lam + k * l[3] - lf) return clamp_k(k);
+    }
+    return clamp_k(floor(lam));
+}
+
 // The first trial of poisson_ptrs as far as its squeeze: true with the count
-// when that accepts.
+// when that accepts; a mean above 2^40 is left to it.
 __device__ __forceinline__ bool poisson_ptrs_quick(double lam, uint32_t wa, uint32_t wb, uint32_t& k_out) {
-    double slam = sqrt(lam);
+    double slam = sqrt_near(lam);
     double b = 0.931 + 2.53 * slam;
     double a = -0.059 + 0.02483 * b;
-    double vr = 0.9277 - 3.6224 / (b - 2.0);
+    double vr = 0.9277 - div_near(3.6224, b - 2.0);
     double U = u32d(wa) - 0.5;
     double V = u32d(wb);
     double us = 0.5 - fabs(U);
-    double k = floor((2.0 * a / us + b) * U + lam + 0.43);
+    double k = floor((div_near(2.0 * a, us) + b) * U + lam + 0.43);
     k_out = clamp_k(k);
-    return us >= 0.07 && V <= vr;
-}
-
-static __device__ uint32_t poisson(double lam, uint32_t wa, uint32_t wb, uint64_t seed, uint32_t tag,
-                            uint32_t step, uint32_t sim, uint32_t odd) {
-    if (lam < 10.0 || !(lam > 0.0)) return poisson_inversion(lam, wa);
-    return poisson_ptrs(lam, wa, wb, seed, tag, step, sim, odd);
+    return lam < 0x1p40 && us >= 0.07 && V <= vr;
 }
 
 // Cao's g_i (tau.cu:1741-1789) in FP32.
@@ -366,6 +471,40 @@ __device__ __forceinline__ float gfun(uint32_t hor, uint32_t hort, int32_t x) {
             return 3.0f;
         default: return 1.0f;
     }
+}
+
+// Cao's bound on the leap for one species (tau.cu:1741-1922): the smaller of
+// m / |mu| and m^2 / sigma^2 with m = max(eps x / g, 1).  sigma^2 is not 0, mu
+// is 0 only where the bound by mu is infinite.
+static __device__ __noinline__ float tau_bound_any(uint32_t hor, uint32_t hort, int32_t x, float eps, float mu, float sg) {
+    const float tmp2 = (eps * (float)x) / gfun(hor, hort, x);
+    const float macs = tmp2 > 1.0f ? tmp2 : 1.0f;
+    const float t3 = mu != 0.0f ? macs / fabsf(mu) : __int_as_float(0x7f800000);
+    const float t4 = (macs * macs) / sg;
+    return t3 < t4 ? t3 : t4;
+}
+__device__ __forceinline__ float tau_bound(uint32_t hor, uint32_t hort, int32_t x, float eps, float mu, float sg) {
+    const float xf = (float)x, ex = eps * xf, d1 = xf - 1.0f, d2 = xf - 2.0f;
+    bool fits = num_fits(ex) & div_fits(mu) & div_fits(sg);
+    float tmp2 = ex;  // g = 1
+    if (hor == 2u || hor == 3u) {
+        float g = hor == 2u ? 2.0f : 3.0f;
+        if (hort >= 2u && hort <= hor) {  // g depends on x
+            fits &= div_fits(d1);
+            if (hort == 3u) {
+                fits &= div_fits(d2);
+                g = 3.0f + div_near(1.0f, d1) + div_near(2.0f, d2);
+            } else {
+                g = g + div_near(hor == 2u ? 1.0f : 1.5f, d1);
+            }
+            fits &= div_fits(g);
+        }
+        tmp2 = div_near(ex, g);
+    }
+    const float macs = tmp2 > 1.0f ? tmp2 : 1.0f;
+    const float t3 = div_near(macs, fabsf(mu)), t4 = div_near(macs * macs, sg);
+    if (!(fits & (macs < 0x1p30f))) return tau_bound_any(hor, hort, x, eps, mu, sg);
+    return t3 < t4 ? t3 : t4;
 }
 
 // One binary level: left unless the target lies beyond a positive left

@@ -419,10 +419,8 @@ static int default_ssa_budget() { return 100; }
 static int default_dec_budget(int G) { return G >= 32 ? 8 : 2; }
 
 // Launch shape of the register-resident sweep for tiny networks: one thread
-// per simulation, `warp_sims` working lanes per warp.  Library choice of
-// warp_sims: spread a small batch so that about 8 warps per SM work (each
-// warp then runs the union of fewer simulations' paths), whole warps once the
-// batch fills them; smaller blocks while the batch would not reach every SM.
+// per simulation, `warp_sims` working lanes per warp; smaller blocks while the
+// batch would not reach every SM.
 struct TinyOcc {
     int dev;
     const void* kernel;
@@ -433,7 +431,18 @@ struct TinyOcc {
 static std::vector<TinyOcc> g_tiny_occ;
 
 // Scheduling of the register-resident sweep when the caller does not choose.
-static constexpr int TINY_DEFAULT_SCHED = 1;
+// A warp steps its simulations together whatever their number, so what counts
+// is how few of them wait for another's leap.  Up to one simulation per
+// resident warp (8 per SM), each has its own warp (600 Schlogl simulations on
+// one B200: 1.04 ms against 1.36 in block rounds).  Up to two blocks of 32 per
+// SM, rounds keep leaps and exact steps in different warps (4,096: 10.5 against
+// 12.4 ms; 8,192: 12.2 against 13.6).  Beyond, issue slots count, and full
+// warps in lockstep waste the fewest (16,384: 15.3 against 16.4 ms; 65,537 with
+// perturbed rates: 73 against 104).  A shape given by the caller keeps rounds.
+static int tiny_sched(const ctl_run_cfg* cfg, uint32_t n, int sm_count) {
+    if (cfg->threads > 0 || cfg->warp_sims > 0) return 1;
+    return (uint64_t)n <= (uint64_t)sm_count * 8 || (uint64_t)n > (uint64_t)sm_count * 64 ? 2 : 1;
+}
 // Block rounds: a block whose queue is closed finishes a lone simulation in
 // warp lockstep (Schlogl's slowest simulation alone: 6.6 ms against 8.8 ms
 // in rounds); with 2 or more the rounds keep their advantage (16,384
@@ -451,7 +460,7 @@ static ctl_status plan_tiny(const HostTables& t, const ctl_run_cfg* cfg, uint32_
     // against 128 with spills at 2) -- 4,096 simulations on one B200: 330k
     // against 295k sims/s; 65,536: 722k against 650k
     const int minb = cfg->min_blocks > 0 ? cfg->min_blocks : 1;
-    const int sched = cfg->sched > 0 ? cfg->sched : TINY_DEFAULT_SCHED;
+    const int sched = cfg->sched > 0 ? cfg->sched : tiny_sched(cfg, n, da.sm_count);
     pl.spec = cfg->spec >= 0 ? tiny_spec_kernel(t, cfg->flags, minb, sched, nullptr) : nullptr;
     const void* k = pl.spec ? pl.spec : tiny_kernel_ptr(pl.tinyP, pl.tinySM);
     if (!k) {
@@ -473,20 +482,23 @@ static ctl_status plan_tiny(const HostTables& t, const ctl_run_cfg* cfg, uint32_
         // a small batch is spread over every SM.
         const uint64_t wpb = (uint64_t)threads / 32;
         if (ws <= 0) {
-            // 8 per warp (16 live simulations in a 64-thread block) measured
-            // best for Schlogl, 4,096 simulations: 291k sims/s against 254k
-            // with 14 (one block per SM) and 239k for warp lockstep
+            // 8 per warp (16 live simulations in a 64-thread block) up to two
+            // blocks per SM, else 16 (Schlogl, 4,096 simulations: 10.5 ms with
+            // 8, 11.4 with 16; 8,192: 15.0 and 12.2)
             const uint64_t per = ((uint64_t)n + (uint64_t)da.sm_count * wpb - 1) / ((uint64_t)da.sm_count * wpb);
-            ws = (int)std::min<uint64_t>(8, std::max<uint64_t>(1, per));
+            ws = per > 16 ? 16 : (int)std::min<uint64_t>(8, std::max<uint64_t>(1, per));
         }
         const uint64_t slots = (uint64_t)ws * wpb;
-        smem = (size_t)(2 * pl.tinySM + 20 + pl.tinyP) * (size_t)threads * 4;  // Packed<P, SM>::WORDS
+        smem = tiny_smem(pl.tinyP, pl.tinySM, threads, 1);
         need = ((uint64_t)n + slots - 1) / slots;
     } else {
         if (ws <= 0) {
-            const uint64_t target_warps = (uint64_t)da.sm_count * 8;
+            // one each while every SM holds them (8 warps), else four warps per
+            // SM before the warps fill (Schlogl, 8,192 simulations: 13.6 ms with
+            // 16, 15.9 with 8; 16,384: 15.3 with 32, 18.6 with 16)
             ws = 1;
-            while (ws < 32 && (uint64_t)n > target_warps * (uint64_t)ws) ws <<= 1;
+            if ((uint64_t)n > (uint64_t)da.sm_count * 8)
+                while (ws < 32 && (uint64_t)n > (uint64_t)da.sm_count * 4 * (uint64_t)ws) ws <<= 1;
         }
         const uint64_t warps = ((uint64_t)n + ws - 1) / ws;
         // a batch of about one wave: blocks of two warps spread it evenly over
@@ -494,6 +506,7 @@ static ctl_status plan_tiny(const HostTables& t, const ctl_run_cfg* cfg, uint32_
         // sims/s with 192-thread blocks, which leave some SMs one block and
         // others two)
         if (cfg->threads <= 0 && warps <= (uint64_t)da.sm_count * 8) threads = 64;
+        smem = tiny_smem(pl.tinyP, pl.tinySM, threads, 2);
         need = (warps * 32 + threads - 1) / threads;
     }
     if (smem > (size_t)da.smem_optin) {
@@ -547,10 +560,12 @@ static ctl_status plan_tiny(const HostTables& t, const ctl_run_cfg* cfg, uint32_
     pl.smem = smem;
     pl.minb = pl.spec ? minb : 2;
     pl.sched = sched;
-    // rounds of 16 SSA steps and 2 decisions for block rounds (a deciding warp
-    // then takes about as long as a stepping one), 16 and 1 in warp lockstep
-    pl.ssa_budget = cfg->ssa_budget > 0 ? cfg->ssa_budget : 16;
-    pl.dec_budget = cfg->dec_budget > 0 ? cfg->dec_budget : (sched == 1 ? 2 : 1);
+    // 64 SSA steps and 4 decisions per block round (a deciding warp then takes
+    // about as long as a stepping one; Schlogl, 4,096 simulations: 10.5 ms, 11.0
+    // with 16 and 2, 10.9 with 128 and 4); in lockstep 16 and 1 (4,096, 8 per
+    // warp: 12.4 ms, 20.0 with 16 and 4)
+    pl.ssa_budget = cfg->ssa_budget > 0 ? cfg->ssa_budget : (sched == 1 ? 64 : 16);
+    pl.dec_budget = cfg->dec_budget > 0 ? cfg->dec_budget : (sched == 1 ? 4 : 1);
     pl.warp_sims = ws;
     return CTL_OK;
 }
@@ -1139,9 +1154,9 @@ extern "C" ctl_status ctl_autotune(ctl_model* m, const ctl_run_cfg* cfg, uint32_
         consider(bestx);                                       // 0. the library's own plan
         if (tiny_eligible(t)) {                                // 1a. register-resident sweep
             for (int ws : {1, 2, 4, 8, 16, 32})                //     warp lockstep
-                if (!(ws == p0.warp_sims && p0.sched == 2)) consider({1, 0, S0 > 0 ? S0 : 16, 1, 1, 2, ws});
+                if (!(ws == p0.warp_sims && p0.sched == 2)) consider({1, 0, cfg->ssa_budget > 0 ? S0 : 16, 1, 1, 2, ws});
             for (int ws : {4, 8, 12, 16})                      //     block rounds with regrouping
-                if (!(ws == p0.warp_sims && p0.sched == 1)) consider({1, 0, S0 > 0 ? S0 : 16, 2, 1, 1, ws});
+                if (!(ws == p0.warp_sims && p0.sched == 1)) consider({1, 0, cfg->ssa_budget > 0 ? S0 : 64, 4, 1, 1, ws});
         }
         for (int G = 1; G <= 256 && G <= t.P; G <<= 1)        // 1b. lanes per simulation
             if (G != p0.G || p0.warp_sims > 0) consider({G, 256, S0, default_dec_budget(G), 2, 1, -1});

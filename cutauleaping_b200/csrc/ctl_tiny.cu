@@ -23,6 +23,7 @@
 #include <dlfcn.h>
 #include <nvrtc.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -78,6 +79,13 @@ bool tiny_eligible(const HostTables& t) {
 }
 
 int tiny_species_bound(const HostTables& t) { return t.S <= 4 ? 4 : 8; }
+
+size_t tiny_smem(int P, int SM, int threads, int sched) {
+    // the warps' areas (Area<P>::BYTES), and for block rounds the exchange (Packed<P, SM>::WORDS per thread)
+    const size_t area = (size_t)tiny::area_bytes(P);
+    return (size_t)(threads / 32) * area + (sched == 1 ? (size_t)(2 * SM + 16 + P) * threads * 4 : 0);
+}
+static_assert(tiny::Packed<4, 8>::WORDS == 2 * 8 + 16 + 4, "tiny_smem and the kernel body agree");
 
 void tiny_net(const HostTables& t, uint32_t flags, const double* d_tvec, tiny::Net& n) {
     std::memset(&n, 0, sizeof(n));
@@ -228,11 +236,9 @@ std::string spec_source(const HostTables& t, uint32_t flags, int minb, int sched
     // one schedule per kernel: warp lockstep (2) or block rounds (1)
     o << "extern \"C\" __global__ void __launch_bounds__(256, " << minb << ") ctl_tiny_spec("
          "const __grid_constant__ NetCT net, const __grid_constant__ ctl::dev::Run run, unsigned lanes) {\n";
-    if (sched == 2)
-        o << "    ctl::tiny::sweep<NetCT, " << P << ", " << SM << ">(net, run, lanes);\n}\n";
-    else
-        o << "    extern __shared__ unsigned ctl_tiny_xs[];\n"
-             "    ctl::tiny::sweep_rounds<NetCT, " << P << ", " << SM << ">(net, run, lanes, ctl_tiny_xs);\n}\n";
+    o << "    extern __shared__ __align__(16) unsigned ctl_tiny_xs[];\n"
+      << (sched == 2 ? "    ctl::tiny::sweep<NetCT, " : "    ctl::tiny::sweep_rounds<NetCT, ") << P << ", " << SM
+      << ">(net, run, lanes, ctl_tiny_xs);\n}\n";
     return o.str();
 }
 

@@ -39,6 +39,9 @@ struct Net {
 bool tiny_eligible(const HostTables& t);
 // Species bound of the kernel variant (4 or 8).
 int tiny_species_bound(const HostTables& t);
+// Dynamic shared memory of a block: P tree leaves, species bound SM, schedule
+// (1 block rounds, 2 warp lockstep).
+size_t tiny_smem(int P, int SM, int threads, int sched);
 // Parameter block for a run with `flags` (quirk Q5 picks the tau1 table).
 void tiny_net(const HostTables& t, uint32_t flags, const double* d_tvec, tiny::Net& n);
 // Kernel for P tree leaves (2, 4, 8, 16) and species bound SM (4, 8).

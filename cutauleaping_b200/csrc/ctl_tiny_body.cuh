@@ -8,7 +8,17 @@
 // One thread owns one simulation and keeps everything in registers:
 // populations, the proposed leap state, rate constants, propensities, the
 // complete FP64 sum tree over the reactions, the Poisson counts and the last
-// recorded sample.  Same arithmetic contract as the shared-memory sweep and
+// recorded sample.  What needs no simulation state is done by the warp: the
+// random parts of a stretch of SSA steps are prepared ahead into shared
+// memory, and the Poisson draws of all its leaping simulations are dealt out
+// over the 32 lanes.  All 32 lanes therefore run every phase together, lanes
+// without work along with the others.  What bounds it is the chain of dependent
+// operations of a step or leap (a batch lasts as long as its slowest
+// simulation): 0.29 us per exact step of a lone Schlogl simulation (0.49 before
+// the random parts were prepared ahead, the sample test moved behind the state
+// update and the divisions became straight-line code), 3.3 us per leap.  One
+// B200: 4,096 simulations 12.7 -> 8.9 ms, 65,537 with perturbed rates 175 -> 71
+// ms, whose slowest takes 9,901 leaps.  Same arithmetic contract as the shared-memory sweep and
 // the CPU oracle (oracle/ctl_oracle.c), bit for bit: Philox4x32-10 counters
 // (seed, block, tag, step, sim), FP32 propensities in the reference's factor
 // order, FP64 sums as the root of the binary tree over P = 2^k leaves and the
@@ -43,6 +53,14 @@ __device__ __forceinline__ int32_t pick(const int32_t (&x)[SM], uint32_t s) {
     return v;
 }
 
+// x / j, correctly rounded, for a normal x and a small integer j > 2, without a
+// division's test and branch: with y = 1 / j rounded to nearest, q = x y and one
+// correction by the exact remainder give the rounded quotient (Markstein 1990).
+__device__ __forceinline__ float div_small(float x, int j) {
+    const float b = (float)j, y = 1.0f / b, q = x * y;
+    return fmaf(fmaf(-b, q, x), y, q);
+}
+
 // Mass-action propensity of reaction r in FP32 (CalculatePropensity,
 // tau.cu:1443-1470): c times, per reactant entry in species order, X
 // (coefficient 1), 0.5 X (X-1) (2) or the running product of (X-j+1)/j
@@ -68,7 +86,7 @@ __device__ __forceinline__ float propensity(const N& net, int r, float c, const 
                 // (x-j+1)/j: division by 1 and 2 is exact scaling, the rest divides
                 v = v * (float)xs;
                 v = v * ((float)(xs - 1) * 0.5f);
-                for (int j = 3; j <= st; j++) v = v * ((float)(xs - j + 1) / (float)j);
+                for (int j = 3; j <= st; j++) v = v * div_small((float)(xs - j + 1), j);
             }
         }
     }
@@ -109,41 +127,52 @@ __device__ __forceinline__ int descend(const double (&t)[2 * P - 1], double x) {
     return idx;
 }
 
-// The Poisson sampler out of line: the leap draws from up to 16 call sites,
-// and one copy of its code keeps the kernel small enough for the
-// instruction cache when many warps run different phases.
-__device__ __noinline__ uint32_t poisson_draw(double lam, uint32_t wa, uint32_t wb, uint64_t seed, uint32_t tag,
-                                              uint32_t step, uint32_t sim, uint32_t odd) {
-    return dev::poisson(lam, wa, wb, seed, tag, step, sim, odd);
-}
-
 struct Sim {
     double T, tl, t_next;
-    unsigned long long fire;
+    unsigned long long fire;  // firings of the leaps
     uint32_t sim, cursor, n, burst, leaps, ssa, rej, status;
     bool in_ssa;
-    // The random part of SSA step `pre`, computed during the step before (it
-    // depends on the counters only, not on the state): the pick uniform and
-    // the log of the waiting-time uniform.
-    uint32_t pre;
-    double pre_u;
-    float pre_lg;
-    uint4 wc;         // Philox block of SSA steps 2 wc_blk, 2 wc_blk + 1 (not carried across rounds)
-    uint32_t wc_blk;
 };
 
-// Pick uniform and waiting-time log of SSA step `step`: one Philox block per
-// two steps, (w0, w1) for even steps and (w2, w3) for odd ones, as
-// dev::ssa_step; the block is kept for the pair's second step.
-__device__ __forceinline__ void ssa_randoms(const dev::Run& run, uint32_t simg, uint32_t step, Sim& st, double& u,
-                                            float& lg) {
-    if (st.wc_blk != (step >> 1)) {
-        st.wc = dev::draw(run.seed, 0u, dev::TAG_SSA, step >> 1, simg);
-        st.wc_blk = step >> 1;
+constexpr uint32_t FULL = 0xffffffffu;
+
+// Shared memory of a warp: the random parts of the next SSA steps of each
+// lane's simulation (pick word, negated log of the waiting-time uniform), or,
+// during a leap, the Poisson means, uniforms and counts by reaction and lane, the
+// reactions sorted by how they are drawn, and the lanes' counters.
+constexpr int AHEAD = 18;  // steps prepared: 9 Philox blocks, 17 steps from an odd one
+__host__ __device__ constexpr int area_bytes(int P) {
+    const int rng = AHEAD * 32 * 8, leap = 32 * P * (8 + 8 + 4 + 4) + 256;
+    return rng > leap ? rng : leap;
+}
+template <int P>
+struct Area {
+    static constexpr int DRAWS = 32 * P, BYTES = area_bytes(P);
+    unsigned char* b;
+    __device__ __forceinline__ uint2& rng(uint32_t k) const {
+        return reinterpret_cast<uint2*>(b)[k * 32u + (threadIdx.x & 31u)];
     }
-    const uint32_t wa = (step & 1u) ? st.wc.z : st.wc.x, wb = (step & 1u) ? st.wc.w : st.wc.y;
-    u = dev::u32d(wa);
-    lg = dev::flog(dev::u24f(wb));
+    __device__ __forceinline__ double* lam() const { return reinterpret_cast<double*>(b); }
+    __device__ __forceinline__ uint2* words() const { return reinterpret_cast<uint2*>(b + DRAWS * 8); }
+    __device__ __forceinline__ uint32_t* k() const { return reinterpret_cast<uint32_t*>(b + DRAWS * 16); }
+    __device__ __forceinline__ uint16_t* list() const { return reinterpret_cast<uint16_t*>(b + DRAWS * 20); }
+    __device__ __forceinline__ uint32_t* sim() const { return reinterpret_cast<uint32_t*>(b + DRAWS * 24); }
+    __device__ __forceinline__ uint32_t* step() const { return sim() + 32; }
+};
+
+// The random parts of SSA steps 2 blk, 2 blk + 1, ... : one Philox block per
+// two steps, (w0, w1) for even steps and (w2, w3) for odd ones, as the
+// shared-memory sweep.  They depend on the counters only; prepared AHEAD at a
+// time, three blocks interleaved, they cost a lone simulation 0.04 us a step
+// instead of 0.18 one step ahead.
+template <int P>
+__device__ __forceinline__ void rng_fill(const dev::Run& run, const Area<P>& w, uint32_t simg, uint32_t blk) {
+#pragma unroll 3
+    for (uint32_t i = 0; i < AHEAD / 2; i++) {
+        const uint4 q = dev::draw(run.seed, 0u, dev::TAG_SSA, blk + i, simg);
+        w.rng(2u * i) = make_uint2(q.x, __float_as_uint(-dev::flog(dev::u24f(q.y))));
+        w.rng(2u * i + 1u) = make_uint2(q.z, __float_as_uint(-dev::flog(dev::u24f(q.w))));
+    }
 }
 
 // One simulation's registers.
@@ -215,23 +244,118 @@ __device__ void finish_zero(const N& net, const dev::Run& run, State<P, SM>& s, 
     cursor = ns;
 }
 
-// PreCalculations (tau.cu:1568-2093) for one simulation in registers: the
-// SSA hand-off decision and, unless it hands off, one Cao tau-leap with
-// critical reactions and negative-population rejection.
+// The Poisson counts K of the leaping lanes (todo) in one pass over the warp:
+// every (lane, reaction) with a positive mean is sorted by how it is drawn --
+// inversion with a mean below 1 or below 10, PTRS -- and the 32 lanes take
+// these in turn, so that a few leaping simulations fill the warp and its lanes
+// run one path at a time; PTRS draws that the squeeze does not accept are
+// collected for the full test.
 template <class N, int P, int SM>
-__device__ int decide_step(const N& net, const dev::Run& run, State<P, SM>& s, Sim& st, const Out& o) {
+__device__ __forceinline__ void poisson_pass(const N& net, const dev::Run& run, const Area<P>& w, const State<P, SM>& s,
+                                             uint32_t crit, uint32_t simg, uint32_t step, uint32_t attempt, double tau,
+                                             int pick_r, bool todo, uint32_t (&K)[P]) {
+    const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+    const bool keep = attempt == 0 || (run.flags & dev::F_Q3_OFF);
+    // means below 1 from the front of the first list, below 10 from its back,
+    // the others in the second list behind it
+    uint16_t *list = w.list(), *large = list + Area<P>::DRAWS;
+    uint32_t nt = 0, nsm = 0, nlg = 0, drawn = 0;
+    __syncwarp();
+    w.sim()[lane] = simg;
+    w.step()[lane] = step;
+#pragma unroll
+    for (int r = 0; r < P; r++) {
+        const bool c = r >= net.R() || ((crit >> r) & 1u);
+        const double lam = c ? 0.0 : tau * (double)s.a[r];
+        K[r] = c && r == pick_r && keep ? 1u : 0u;
+        const bool on = todo & (lam > 0.0);
+        const bool ti = on & (lam < 1.0), lg = on & !(lam < 10.0), sm = on & !ti & !lg;
+        const uint32_t bt = __ballot_sync(FULL, ti), bs = __ballot_sync(FULL, sm), bl = __ballot_sync(FULL, lg);
+        const uint32_t e = (uint32_t)(r * 32) + lane;
+        const uint32_t at = ti ? nt + __popc(bt & below)
+                               : sm ? Area<P>::DRAWS - 1u - nsm - __popc(bs & below) : Area<P>::DRAWS + nlg + __popc(bl & below);
+        w.lam()[e] = lam;
+        if (on) list[at] = (uint16_t)e;
+        drawn |= on ? 1u << r : 0u;
+        nt += __popc(bt);
+        nsm += __popc(bs);
+        nlg += __popc(bl);
+    }
+    // the uniforms: a block per pair of reactions, by the lane that holds the simulation
+#pragma unroll 2
+    for (int r = 0; r < P; r += 2) {
+        const uint4 q = dev::draw_small(run.seed, 0u, dev::tag_pois(attempt, (uint32_t)r >> 1), step, simg);
+        w.words()[r * 32 + (int)lane] = make_uint2(q.x, q.y);
+        if (P > 1) w.words()[r * 32 + 32 + (int)lane] = make_uint2(q.z, q.w);
+    }
+    __syncwarp();
+#pragma unroll 1
+    for (int part = 0; part < 2; part++) {
+        const uint32_t n = part ? nsm : nt;
+#pragma unroll 1
+        for (uint32_t i = lane; i < n; i += 32u) {
+            const uint32_t e = list[part ? Area<P>::DRAWS - 1 - (int)i : (int)i];
+            w.k()[e] = dev::poisson_inversion(w.lam()[e], w.words()[e].x);
+        }
+    }
+    uint32_t nslow = 0;
+#pragma unroll 1
+    for (uint32_t i0 = 0; i0 < nlg; i0 += 32u) {
+        bool slow = false;
+        uint32_t e = 0;
+        if (i0 + lane < nlg) {
+            e = large[i0 + lane];
+            const uint2 q = w.words()[e];
+            uint32_t k;
+            slow = !dev::poisson_ptrs_quick(w.lam()[e], q.x, q.y, k);
+            if (!slow) w.k()[e] = k;
+        }
+        const uint32_t b = __ballot_sync(FULL, slow);  // also orders the reads above before the writes below
+        if (slow) large[nslow + __popc(b & below)] = (uint16_t)e;
+        nslow += __popc(b);
+    }
+    __syncwarp();
+#pragma unroll 1
+    for (uint32_t i = lane; i < nslow; i += 32u) {
+        const uint32_t e = large[i];
+        const uint2 q = w.words()[e];
+        w.k()[e] = dev::poisson_ptrs_wide(w.lam()[e], q.x, q.y, run.seed, dev::tag_pois(attempt, e >> 6), w.step()[e & 31u],
+                                     w.sim()[e & 31u], (e >> 5) & 1u);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < P; r++)
+        if ((drawn >> r) & 1u) K[r] = w.k()[r * 32 + (int)lane];
+}
+
+// PreCalculations (tau.cu:1568-2093) for the lanes with act: the SSA hand-off
+// decision and, unless it hands off, one Cao tau-leap with critical reactions
+// and negative-population rejection.
+template <class N, int P, int SM>
+__device__ __forceinline__ int decide_step(const N& net, const dev::Run& run, const Area<P>& w, State<P, SM>& s, Sim& st,
+                                           const Out& o, bool act) {
     const uint32_t fl = run.flags;
     const uint32_t ns = (uint32_t)net.ns();
     const int so = net.s_out();
     const uint32_t simg = run.sim_base + st.sim;
-    if (st.T >= net.tmax()) return DONE;
-    if (st.n >= run.max_steps) { st.status = CTL_SIM_STEP_LIMIT; return DONE; }
-    const uint32_t step = st.n++;
+    const uint32_t step = st.n;
     const double A0 = s.t[2 * P - 2];
-    if (A0 == 0.0) {
-        finish_zero<N, P, SM>(net, run, s, o, st.cursor);
-        st.T = net.tmax() + (double)0.1f;
-        return DONE;
+    int res = CONT;
+    if (act) {
+        if (st.T >= net.tmax()) {
+            res = DONE;
+        } else if (step >= run.max_steps) {
+            st.status = CTL_SIM_STEP_LIMIT;
+            res = DONE;
+        } else {
+            st.n = step + 1u;
+            if (A0 == 0.0) {
+                finish_zero<N, P, SM>(net, run, s, o, st.cursor);
+                st.T = net.tmax() + (double)0.1f;
+                res = DONE;
+            }
+        }
+        act = res == CONT;
     }
     // critical reactions (tau.cu:1727-1733): some reactant with
     // 0 < floor(x / L) < n_c, tested as x >= L and x < n_c L
@@ -245,7 +369,7 @@ __device__ int decide_step(const N& net, const dev::Run& run, State<P, SM>& s, S
             if (r < net.R() && e < (int)net.ne(r)) {
                 const uint32_t xs = (uint32_t)pick<SM>(s.x, net.es(r, e)), L = net.ec(r, e);
                 const bool below = (uint64_t)xs < (uint64_t)run.nc * L;
-                cr = cr || (q6off ? below : (xs >= L && below));
+                cr = cr | (below & (q6off | (xs >= L)));
             }
         }
         crit |= cr ? (1u << r) : 0u;
@@ -268,200 +392,218 @@ __device__ int decide_step(const N& net, const dev::Run& run, State<P, SM>& s, S
                 }
             }
             const int32_t xs = s.x[q];
-            const float gg = dev::gfun(net.hor(q), net.hort(q), xs);
-            const float tmp2 = (run.eps * (float)xs) / gg;
-            const float macs = tmp2 > 1.0f ? tmp2 : 1.0f;
             const bool use = (fl & dev::F_Q9_OFF) ? (sg != 0.0f) : (mu != 0.0f && sg != 0.0f);
             if (use) {
-                const float t3 = mu != 0.0f ? macs / fabsf(mu) : __int_as_float(0x7f800000);
-                const float t4 = (macs * macs) / sg;
-                const float tt = t3 < t4 ? t3 : t4;
+                const float tt = dev::tau_bound(net.hor(q), net.hort(q), xs, run.eps, mu, sg);
                 if (tt < tau1) tau1 = tt;
             }
         }
     }
-    if ((double)tau1 < run.ssa_factor / A0) {
+    if (act && (double)tau1 < run.ssa_factor / A0) {
         st.in_ssa = true;
         st.burst = 0;
         st.tl = 0.0;
-        return CONT;
+        act = false;
     }
-    double tc[2 * P - 1];  // critical tree
-    double a0c = 0.0;
-    if (crit) {
+    if (!__any_sync(FULL, act)) return res;  // from here on only the leaping lanes
+    double tau = (double)tau1;
+    int pick_r = -1;
+    if (act && crit) {
+        double tc[2 * P - 1];  // critical tree
 #pragma unroll
         for (int r = 0; r < P; r++) tc[r] = (crit >> r) & 1u ? (double)s.a[r] : 0.0;
         build<P>(tc);
-        a0c = tc[2 * P - 2];
-    }
-    double tau2 = (double)FLT_MAX;
-    int pick_r = -1;
-    if (a0c > 0.0) {  // the draw serves tau2 and the critical pick only
-        const uint4 wd = dev::draw(run.seed, 0u, dev::TAG_MISC, step, simg);
-        tau2 = -dev::dlog(dev::u53(wd.x, wd.y)) / a0c;
-        if ((double)tau1 > tau2) {
-            // the reference's linear search starts from PROP[0] unmasked (Q2):
-            // leaf 0 joins the tree when it is not critical itself
-            if (!(fl & dev::F_Q2_OFF) && !(crit & 1u)) {
-                tc[0] = (double)s.a[0];
-                build<P>(tc);
+        const double a0c = tc[2 * P - 2];
+        if (a0c > 0.0) {  // the draw serves tau2 and the critical pick only
+            const uint4 wd = dev::draw_small(run.seed, 0u, dev::TAG_MISC, step, simg);
+            const double tau2 = -dev::dlog(dev::u53(wd.x, wd.y)) / a0c;
+            if ((double)tau1 > tau2) {
+                // the reference's linear search starts from PROP[0] unmasked (Q2):
+                // leaf 0 joins the tree when it is not critical itself
+                if (!(fl & dev::F_Q2_OFF) && !(crit & 1u)) {
+                    tc[0] = (double)s.a[0];
+                    build<P>(tc);
+                }
+                pick_r = descend<P>(tc, dev::u53(wd.z, wd.w) * a0c);
+                tau = tau2;
             }
-            pick_r = descend<P>(tc, dev::u53(wd.z, wd.w) * a0c);
         }
     }
-    double tau = (double)tau1 < tau2 ? (double)tau1 : tau2;
-    uint32_t attempt = 0;
     uint32_t K[P];
     int32_t x1[SM];
-    bool ovf = false;
-    for (;;) {
-        const bool keep = attempt == 0 || (fl & dev::F_Q3_OFF);
+    bool todo = act;
+    for (uint32_t attempt = 0;; attempt++) {
+        uint32_t Kn[P];
+        poisson_pass<N, P, SM>(net, run, w, s, crit, simg, step, attempt, tau, pick_r, todo, Kn);
+        if (todo) {
+            // test_update (tau.cu:1300-1351): entries of F species-major in
+            // ascending reaction order, rejected at the first negative (Q4)
+            const bool every = !(fl & dev::F_Q4_OFF);
+            bool fail = false, lovf = false;
 #pragma unroll
-        for (int pb = 0; 2 * pb < P; pb++) {
-            const int r0 = 2 * pb, r1 = r0 + 1;
-            const bool c0 = r0 >= net.R() || ((crit >> r0) & 1u);
-            const bool c1 = r1 >= net.R() || ((crit >> r1) & 1u);
-            const double l0 = c0 ? 0.0 : tau * (double)s.a[r0];
-            const double l1 = c1 ? 0.0 : tau * (double)s.a[r1];
-            const uint32_t tg = dev::tag_pois(attempt, (uint32_t)pb);
-            uint4 w = make_uint4(0u, 0u, 0u, 0u);
-            if (l0 > 0.0 || l1 > 0.0) w = dev::draw(run.seed, 0u, tg, step, simg);
-            K[r0] = c0 ? ((r0 == pick_r && keep) ? 1u : 0u) : poisson_draw(l0, w.x, w.y, run.seed, tg, step, simg, 0u);
-            K[r1] = c1 ? ((r1 == pick_r && keep) ? 1u : 0u) : poisson_draw(l1, w.z, w.w, run.seed, tg, step, simg, 1u);
-        }
-        // test_update (tau.cu:1300-1351): entries of F species-major in
-        // ascending reaction order, rejected at the first negative (Q4)
-        bool fail = false, lovf = false;
+            for (int r = 0; r < P; r++) K[r] = Kn[r];
 #pragma unroll
-        for (int q = 0; q < SM; q++) {
-            int64_t v = s.x[q];
-            bool neg = false;
+            for (int q = 0; q < SM; q++) {
+                int64_t v = s.x[q];
 #pragma unroll
-            for (int r = 0; r < P; r++) {
-                const int f = (q < net.S() && r < net.R()) ? (int)net.Fm(q, r) : 0;
-                if (f != 0 && !neg) {
-                    v += (int64_t)f * (int64_t)K[r];
-                    if (!(fl & dev::F_Q4_OFF) && v < 0) neg = true;
+                for (int r = 0; r < P; r++) {
+                    const int f = (q < net.S() && r < net.R()) ? (int)net.Fm(q, r) : 0;
+                    if (f != 0) {
+                        v += (int64_t)f * (int64_t)(int32_t)K[r];
+                        fail |= (v < 0) & every;
+                    }
                 }
+                fail |= v < 0;
+                lovf |= v > 2147483647LL;
+                x1[q] = (int32_t)v;
             }
-            if (neg || v < 0) fail = true;
-            if (v > 2147483647LL) lovf = true;
-            x1[q] = (int32_t)v;
+            todo = fail;
+            if (fail) {
+                tau = tau * 0.5;
+                st.rej++;
+                if (attempt + 1u >= dev::MAX_ATTEMPTS) {
+                    st.status = CTL_SIM_ATTEMPT_LIMIT;
+                    res = DONE;
+                    act = todo = false;
+                }
+            } else if (lovf) {
+                st.status = CTL_SIM_OVERFLOW;
+                res = DONE;
+                act = false;
+            }
         }
-        if (!fail) {
-            ovf = lovf;
-            break;
-        }
-        tau = tau * 0.5;
-        attempt++;
-        st.rej++;
-        if (attempt >= dev::MAX_ATTEMPTS) { st.status = CTL_SIM_ATTEMPT_LIMIT; return DONE; }
+        if (!__any_sync(FULL, todo)) break;
     }
-    if (ovf) { st.status = CTL_SIM_OVERFLOW; return DONE; }
-    // check_time_instant (tau.cu:1507-1562)
-    const double T = st.T;
-    while (st.cursor < ns && T + tau >= st.t_next) {
-        for (int k = 0; k < so; k++) {
-            const uint32_t sp = net.cs(k);
-            const int32_t xs = pick<SM>(s.x, sp);
-            const double d = (double)((int64_t)pick<SM>(x1, sp) - (int64_t)xs);
-            const double delta = (d * (st.t_next - T)) / tau;
-            const double ri = rint(delta);
-            uint32_t v;
-            if (!(fl & dev::F_Q1_OFF)) v = (uint32_t)xs + (ri > 0.0 ? (uint32_t)ri : 0u);
-            else v = (uint32_t)((int64_t)xs + (int64_t)ri);
-            put<P, SM>(o, s, st.cursor, so, k, v);
+    if (act) {
+        // check_time_instant (tau.cu:1507-1562)
+        const double T = st.T;
+        while (st.cursor < ns && T + tau >= st.t_next) {
+            for (int k = 0; k < so; k++) {
+                const uint32_t sp = net.cs(k);
+                const int32_t xs = pick<SM>(s.x, sp);
+                const double d = (double)((int64_t)pick<SM>(x1, sp) - (int64_t)xs);
+                const double delta = (d * (st.t_next - T)) / tau;
+                const double ri = rint(delta);
+                uint32_t v;
+                if (!(fl & dev::F_Q1_OFF)) v = (uint32_t)xs + (ri > 0.0 ? (uint32_t)ri : 0u);
+                else v = (uint32_t)((int64_t)xs + (int64_t)ri);
+                put<P, SM>(o, s, st.cursor, so, k, v);
+            }
+            st.cursor++;
+            st.t_next = st.cursor < ns ? net.tvec()[st.cursor] : 0.0;
         }
-        st.cursor++;
-        st.t_next = st.cursor < ns ? net.tvec()[st.cursor] : 0.0;
+        unsigned long long fs = 0;
+#pragma unroll
+        for (int r = 0; r < P; r++) fs += K[r];
+        st.fire += fs;
+        st.leaps++;
+#pragma unroll
+        for (int q = 0; q < SM; q++) s.x[q] = x1[q];
+        st.T = T + tau;
+        all_props<N, P, SM>(net, s);
+        if (st.cursor == ns) res = DONE;
     }
-    unsigned long long fs = 0;
-#pragma unroll
-    for (int r = 0; r < P; r++) fs += K[r];
-    st.fire += fs;
-    st.leaps++;
-#pragma unroll
-    for (int q = 0; q < SM; q++) s.x[q] = x1[q];
-    st.T = T + tau;
-    all_props<N, P, SM>(net, s);
-    return st.cursor == ns ? DONE : CONT;
+    return res;
 }
 
-// EventualSSASteps / LightweightSSA (tau.cu:2099-2454): one direct-method
-// step.
-template <class N, int P, int SM>
-__device__ __forceinline__ int ssa_step(const N& net, const dev::Run& run, State<P, SM>& s, Sim& st,
-                                        const Out& o) {
+// Entry j of a row of F from the word that holds it.
+__device__ __forceinline__ int32_t net_change(uint32_t word, int j) {
+    return (int32_t)(int8_t)(uint8_t)(word >> (8 * (j & 3)));
+}
+
+// EventualSSASteps / LightweightSSA (tau.cu:2099-2454): direct-method steps of
+// the lanes with `act` (which hold a simulation in its SSA phase) while
+// more(b) holds for step number b.  A step is straight-line code for all
+// lanes: one that may not step any more changes nothing (F = 0); what rarely
+// happens -- a sample instant, the end of a burst, a limit -- waits in one
+// branch each.
+template <class N, int P, int SM, class More>
+__device__ __forceinline__ int ssa_steps(const N& net, const dev::Run& run, const Area<P>& w, State<P, SM>& s, Sim& st,
+                                         const Out& o, bool act, More&& more) {
     const uint32_t ns = (uint32_t)net.ns();
     const int so = net.s_out();
-    if (st.n >= run.max_steps) { st.status = CTL_SIM_STEP_LIMIT; return DONE; }
-    const double A0 = s.t[2 * P - 2];
-    if (A0 == 0.0) {
-        finish_zero<N, P, SM>(net, run, s, o, st.cursor);
-        st.T = net.tmax() + (double)0.1f;
-        return DONE;
-    }
-    const uint32_t step = st.n++;
-    const uint32_t simg = run.sim_base + st.sim;
-    double u;
-    float lg;
-    if (st.pre == step) {
-        u = st.pre_u;
-        lg = st.pre_lg;
-    } else {
-        ssa_randoms(run, simg, step, st, u, lg);
-    }
-    const int r = descend<P>(s.t, u * A0);
-    // the next step's random part, free of the state (a leap decision in
-    // between leaves it unused)
-    ssa_randoms(run, simg, step + 1u, st, st.pre_u, st.pre_lg);
-    st.pre = step + 1u;
-    const float dtf = -lg / (float)A0;
-    st.tl = st.tl + (double)dtf;
-    while (st.cursor < ns && st.T + st.tl > st.t_next) {
-        for (int k = 0; k < so; k++) put<P, SM>(o, s, st.cursor, so, k, (uint32_t)pick<SM>(s.x, net.cs(k)));
-        st.cursor++;
-        st.t_next = st.cursor < ns ? net.tvec()[st.cursor] : 0.0;
-    }
-    // row r of F: selects over the warp-uniform rows (no memory access)
-    uint32_t f0 = net.frow(0, 0), f1 = net.frow(0, 1);
+    int res = CONT;
+    uint32_t base = 0, left = 0;  // first step prepared, steps until the next preparation
+    for (uint32_t b = 0; __any_sync(FULL, act & more(b)); b++) {
+        if (left == 0u) {
+            base = st.n & ~1u;
+            __syncwarp();
+            rng_fill<P>(run, w, run.sim_base + st.sim, base >> 1);
+            left = AHEAD - 1;
+        }
+        left--;
+        const double A0 = s.t[2 * P - 2];
+        const bool ok = act & (st.n < run.max_steps) & (A0 != 0.0);
+        const uint32_t k = st.n - base;
+        const uint2 q = w.rng(k < (uint32_t)AHEAD ? k : 0u);
+        const int r = descend<P>(s.t, dev::u32d(q.x) * A0);
+        const float lg = __uint_as_float(q.y), a0 = (float)A0;
+        const bool odd = !dev::div_fits(a0);
+        const double tl0 = st.tl;
+        double tl = tl0 + (double)dev::div_near(lg, a0);
+        // row r of F: selects over the warp-uniform rows (no memory access)
+        uint32_t f0 = net.frow(0, 0), f1 = net.frow(0, 1);
 #pragma unroll
-    for (int rr = 1; rr < P; rr++) {
-        f0 = r == rr ? net.frow(rr, 0) : f0;
-        if (SM > 4) f1 = r == rr ? net.frow(rr, 1) : f1;
-    }
-    bool ovf = false;
+        for (int rr = 1; rr < P; rr++) {
+            f0 = r == rr ? net.frow(rr, 0) : f0;
+            if (SM > 4) f1 = r == rr ? net.frow(rr, 1) : f1;
+        }
+        f0 = ok ? f0 : 0u;
+        f1 = ok ? f1 : 0u;
+        // |change| <= 127: the sum wraps negative exactly when it leaves [0, 2^31)
+        int32_t low = 0;
 #pragma unroll
-    for (int q = 0; q < SM; q++) {
-        const uint32_t word = q < 4 ? f0 : f1;
-        const int f = (int)(int8_t)(uint8_t)(word >> (8 * (q & 3)));
-        const int64_t nx = (int64_t)s.x[q] + (int64_t)f;
-        if (f != 0 && (nx > 2147483647LL || nx < 0)) ovf = true;
-        s.x[q] = (int32_t)nx;
+        for (int j = 0; j < SM; j++) {
+            s.x[j] = (int32_t)((uint32_t)s.x[j] + (uint32_t)net_change(j < 4 ? f0 : f1, j));
+            low |= s.x[j];
+        }
+        st.tl = ok ? tl : st.tl;
+        st.n += ok ? 1u : 0u;
+        st.ssa += ok ? 1u : 0u;
+        st.burst += ok ? 1u : 0u;
+        all_props<N, P, SM>(net, s);
+        bool due = ok & (st.T + tl > st.t_next) & (st.cursor < ns);
+        if (act & (!ok | odd | due | (low < 0) | (st.cursor == ns) | (st.burst == run.ssa_steps))) {
+            if (ok & odd) {
+                st.tl = tl = tl0 + (double)(lg / a0);
+                due = (st.T + tl > st.t_next) & (st.cursor < ns);
+            }
+            if (due) {  // the populations before this step
+                int32_t x0[SM];
+#pragma unroll
+                for (int j = 0; j < SM; j++) x0[j] = (int32_t)((uint32_t)s.x[j] - (uint32_t)net_change(j < 4 ? f0 : f1, j));
+                do {
+                    for (int j = 0; j < so; j++) put<P, SM>(o, s, st.cursor, so, j, (uint32_t)pick<SM>(x0, net.cs(j)));
+                    st.cursor++;
+                    st.t_next = st.cursor < ns ? net.tvec()[st.cursor] : 0.0;
+                } while (st.cursor < ns && st.T + tl > st.t_next);
+            }
+            if (!ok) {
+                if (st.n >= run.max_steps) {
+                    st.status = CTL_SIM_STEP_LIMIT;
+                } else {
+                    finish_zero<N, P, SM>(net, run, s, o, st.cursor);
+                    st.T = net.tmax() + (double)0.1f;
+                }
+                res = DONE;
+            } else if (low < 0) {
+                st.status = CTL_SIM_OVERFLOW;
+                res = DONE;
+            } else if (st.cursor == ns) {
+                res = DONE;
+            } else if (st.burst == run.ssa_steps) {
+                st.T = st.T + st.tl;
+                st.tl = 0.0;
+                st.burst = 0;
+                if (!(run.flags & dev::F_FORCE_SSA)) st.in_ssa = false;
+                else if (st.T >= net.tmax()) res = DONE;
+            }
+            act = res == CONT && st.in_ssa;
+        }
     }
-    st.ssa++;
-    st.fire += 1ull;
-    // straight-line from the update to the new sum tree (after an overflow
-    // the propensities are computed and discarded)
-    all_props<N, P, SM>(net, s);
-    if (ovf) { st.status = CTL_SIM_OVERFLOW; return DONE; }
-    st.burst++;
-    if (st.cursor == ns) return DONE;
-    if (st.burst == run.ssa_steps) {
-        st.T = st.T + st.tl;
-        st.tl = 0.0;
-        st.burst = 0;
-        if (!(run.flags & dev::F_FORCE_SSA)) st.in_ssa = false;
-        else if (st.T >= net.tmax()) return DONE;
-    }
-    return CONT;
+    return res;
 }
 
-// One thread per simulation, `lanes` simulations per warp (lanes 0..lanes-1
-// of every warp work, the rest exit), simulations pulled from the device
-// work queue.  The working lanes of a warp take their SSA steps and their
-// leap decisions in lockstep phases (up to ssa_budget SSA steps, then up to
-// dec_budget decisions) so that their instruction streams stay merged.
 // Where simulation `sim` records its samples.
 __device__ __forceinline__ Out out_for(const dev::Run& run, uint32_t sim, size_t row_words) {
     Out o;
@@ -505,8 +647,6 @@ __device__ __forceinline__ void start_sim(const N& net, const dev::Run& run, Sta
     st.cursor = st.n = st.burst = st.leaps = st.ssa = st.rej = 0u;
     st.status = CTL_SIM_OK;
     st.in_ssa = (run.flags & dev::F_FORCE_SSA) != 0;
-    st.pre = 0xffffffffu;
-    st.wc_blk = 0xffffffffu;
 }
 
 template <class N>
@@ -523,7 +663,7 @@ __device__ __forceinline__ void finish(const N& net, const dev::Run& run, const 
             for (int k = 0; k < net.s_out(); k++) o.samples[(size_t)i * net.s_out() + k] = 0u;
     ctl_sim_info inf;
     inf.t_final = st.T + st.tl;
-    inf.firings = st.fire;
+    inf.firings = st.fire + st.ssa;  // every SSA step fires one reaction
     inf.status = st.status;
     inf.steps = st.n;
     inf.leaps = st.leaps;
@@ -548,17 +688,30 @@ __device__ __forceinline__ void finish(const N& net, const dev::Run& run, const 
     }
 }
 
-// Warp lockstep over the lanes of `mask`: each lane steps its simulation (if
-// `live`) and, when it ends, takes the next one from the device work queue,
-// until no lane has one.  The lanes take their SSA steps and their leap
-// decisions in lockstep phases (up to ssa_budget SSA steps, then up to
-// dec_budget decisions) so that their instruction streams stay merged; a
-// lane in one phase waits while the others run the other.
+// No simulation in this lane: values that the phases can run along on.
+template <int P, int SM>
+__device__ __forceinline__ void idle(State<P, SM>& s, Sim& st) {
+#pragma unroll
+    for (int q = 0; q < SM; q++) {
+        s.x[q] = 0;
+        s.last[q] = 0u;
+    }
+#pragma unroll
+    for (int r = 0; r < P; r++) s.c[r] = s.a[r] = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 2 * P - 1; i++) s.t[i] = 0.0;
+    st = Sim{};
+}
+
+// Warp lockstep: each lane steps its simulation (if `live`) and, when it ends,
+// takes the next one from the device work queue (unless `closed`), until no
+// lane has one.  The lanes take their SSA steps and their leap decisions in
+// phases (up to ssa_budget SSA steps, then up to dec_budget decisions); a lane
+// in one phase waits while the others run the other.
 template <class N, int P, int SM>
-__device__ __forceinline__ void lockstep(const N& net, const dev::Run& run, uint32_t mask, State<P, SM>& s, Sim& st,
-                                         Out& o, bool live) {
+__device__ __forceinline__ void lockstep(const N& net, const dev::Run& run, const Area<P>& w, State<P, SM>& s, Sim& st,
+                                         Out& o, bool live, bool closed) {
     const size_t row_words = (size_t)net.ns() * (size_t)net.s_out();
-    bool closed = false;
     for (;;) {
         if (!live && !closed) {
             const uint32_t sim = atomicAdd(run.queue, 1u);
@@ -570,17 +723,14 @@ __device__ __forceinline__ void lockstep(const N& net, const dev::Run& run, uint
                 live = true;
             }
         }
-        if (__all_sync(mask, closed)) break;
-        int res = CONT;
-        for (uint32_t b = 0; b < run.ssa_budget; b++) {
-            const bool act = live && res == CONT && st.in_ssa;
-            if (!__any_sync(mask, act)) break;
-            if (act) res = ssa_step<N, P, SM>(net, run, s, st, o);
-        }
+        if (!__any_sync(FULL, live)) break;
+        int res = ssa_steps<N, P, SM>(net, run, w, s, st, o, live && st.in_ssa,
+                                      [&](uint32_t b) { return b < run.ssa_budget; });
         for (uint32_t b = 0; b < run.dec_budget; b++) {
             const bool act = live && res == CONT && !st.in_ssa;
-            if (!__any_sync(mask, act)) break;
-            if (act) res = decide_step<N, P, SM>(net, run, s, st, o);
+            if (!__any_sync(FULL, act)) break;
+            const int x = decide_step<N, P, SM>(net, run, w, s, st, o, act);
+            res = act ? x : res;
         }
         if (live && res == DONE) {
             finish<N>(net, run, st, o);
@@ -590,30 +740,28 @@ __device__ __forceinline__ void lockstep(const N& net, const dev::Run& run, uint
 }
 
 // Warp lockstep sweep: one thread per simulation, `lanes` simulations per
-// warp (lanes 0..lanes-1 of every warp work, the rest exit), simulations
-// pulled from the device work queue.
+// warp (lanes 0..lanes-1 hold them, the rest only take part in the warp's
+// work), simulations pulled from the device work queue.
 template <class N, int P, int SM>
-__device__ __forceinline__ void sweep(const N& net, const dev::Run& run, uint32_t lanes) {
+__device__ __forceinline__ void sweep(const N& net, const dev::Run& run, uint32_t lanes, uint32_t* xs) {
     const uint32_t lane = threadIdx.x & 31u;
-    if (lane >= lanes) return;
-    const uint32_t mask = lanes >= 32 ? 0xffffffffu : ((1u << lanes) - 1u);
+    const Area<P> w{reinterpret_cast<unsigned char*>(xs) + (threadIdx.x >> 5) * Area<P>::BYTES};
     State<P, SM> s;
     Sim st;
     Out o{nullptr, nullptr};
-    lockstep<N, P, SM>(net, run, mask, s, st, o, false);
+    idle<P, SM>(s, st);
+    lockstep<N, P, SM>(net, run, w, s, st, o, false, lane >= lanes);
 }
 
 // Words of one simulation's resumable state in the regrouping exchange:
-// populations, the time and counters, the next sample instant, the prepared
-// random part of the next SSA step, (fitness mode) the last recorded sample
-// and the rate constants.  Propensities and the sum tree are rebuilt from
+// populations, the time and counters, the next sample instant, (fitness mode)
+// the last recorded sample and the rate constants.  Propensities and the sum tree are rebuilt from
 // them.
 template <int P, int SM>
 struct Packed {
     static constexpr int X = 0, T = SM, TL = SM + 2, FIRE = SM + 4, SIM = SM + 6, CURSOR = SM + 7, NSTEP = SM + 8,
                          BURST = SM + 9, LEAPS = SM + 10, SSA = SM + 11, REJ = SM + 12, FLAGS = SM + 13,
-                         PRE = SM + 14, PREU = SM + 15, PRELG = SM + 17, TNEXT = SM + 18, LAST = SM + 20,
-                         C = 2 * SM + 20, WORDS = 2 * SM + 20 + P;
+                         TNEXT = SM + 14, LAST = SM + 16, C = 2 * SM + 16, WORDS = 2 * SM + 16 + P;
 };
 
 // Word w of slot j: structure of arrays, consecutive slots in consecutive banks.
@@ -642,9 +790,6 @@ __device__ __forceinline__ void put_state(uint32_t* xs, uint32_t ns, uint32_t j,
     w(K::SSA, st.ssa);
     w(K::REJ, st.rej);
     w(K::FLAGS, (st.status << 1) | (st.in_ssa ? 1u : 0u));
-    w(K::PRE, st.pre);
-    w64(K::PREU, (unsigned long long)__double_as_longlong(st.pre_u));
-    w(K::PRELG, __float_as_uint(st.pre_lg));
     w64(K::TNEXT, (unsigned long long)__double_as_longlong(st.t_next));
 #pragma unroll
     for (int r = 0; r < P; r++) w(K::C + r, __float_as_uint(s.c[r]));
@@ -674,11 +819,7 @@ __device__ __forceinline__ void get_state(const N& net, const uint32_t* xs, uint
     const uint32_t f = r(K::FLAGS);
     st.status = f >> 1;
     st.in_ssa = (f & 1u) != 0;
-    st.pre = r(K::PRE);
-    st.pre_u = __longlong_as_double((long long)r64(K::PREU));
-    st.pre_lg = __uint_as_float(r(K::PRELG));
     st.t_next = __longlong_as_double((long long)r64(K::TNEXT));
-    st.wc_blk = 0xffffffffu;
 #pragma unroll
     for (int q = 0; q < P; q++) s.c[q] = __uint_as_float(r(K::C + q));
 }
@@ -697,7 +838,7 @@ __device__ __forceinline__ void get_state(const N& net, const uint32_t* xs, uint
 // which finishes them in warp lockstep with no further barriers or state
 // exchange (a lone simulation steps about a third faster so) while the other
 // warps leave.  xs: dynamic shared memory of Packed<P, SM>::WORDS words per
-// thread.
+// thread, then an Area<P> per warp.
 template <class N, int P, int SM>
 __device__ __forceinline__ void sweep_rounds(const N& net, const dev::Run& run, uint32_t slots, uint32_t* xs) {
     __shared__ uint32_t s_cnt[2][32];
@@ -712,9 +853,12 @@ __device__ __forceinline__ void sweep_rounds(const N& net, const dev::Run& run, 
     const uint32_t nt = blockDim.x, nw = nt >> 5;
     const uint32_t below = (1u << lane) - 1u;
     const size_t row_words = (size_t)net.ns() * (size_t)net.s_out();
+    const Area<P> w{reinterpret_cast<unsigned char*>(xs) + (size_t)Packed<P, SM>::WORDS * nt * 4 +
+                    (size_t)warp * Area<P>::BYTES};
     State<P, SM> s;
     Sim st;
     Out o{nullptr, nullptr};
+    idle<P, SM>(s, st);
     bool live = false;
     if (tid == 0) s_closed = 0u;
     __syncthreads();
@@ -738,9 +882,9 @@ __device__ __forceinline__ void sweep_rounds(const N& net, const dev::Run& run, 
         }
         __syncthreads();
         uint32_t nssa = 0, ndec = 0, offs = 0, offd = 0;
-        for (uint32_t w = 0; w < nw; w++) {
-            const uint32_t a = s_cnt[0][w], b = s_cnt[1][w];
-            if (w < warp) {
+        for (uint32_t i = 0; i < nw; i++) {
+            const uint32_t a = s_cnt[0][i], b = s_cnt[1][i];
+            if (i < warp) {
                 offs += a;
                 offd += b;
             }
@@ -756,11 +900,14 @@ __device__ __forceinline__ void sweep_rounds(const N& net, const dev::Run& run, 
             }
             __syncthreads();
             const uint32_t k = nssa + ndec;
-            if (tid >= k) return;
-            get_state<N, P, SM>(net, xs, nt, tid, s, st);
-            all_props<N, P, SM>(net, s);
-            o = out_for(run, st.sim, row_words);
-            lockstep<N, P, SM>(net, run, k >= 32u ? 0xffffffffu : (1u << k) - 1u, s, st, o, true);
+            if (warp != 0u) return;
+            live = tid < k;
+            if (live) {
+                get_state<N, P, SM>(net, xs, nt, tid, s, st);
+                all_props<N, P, SM>(net, s);
+                o = out_for(run, st.sim, row_words);
+            }
+            lockstep<N, P, SM>(net, run, w, s, st, o, live, true);
             return;
         }
         // the other parity's flags were last read in the round before this one
@@ -788,36 +935,32 @@ __device__ __forceinline__ void sweep_rounds(const N& net, const dev::Run& run, 
             all_props<N, P, SM>(net, s);
             o = out_for(run, st.sim, row_words);
         }
-        const uint32_t smask = __ballot_sync(0xffffffffu, mine_ssa);
-        const uint32_t dmask = __ballot_sync(0xffffffffu, mine_dec);
-        int res = CONT;
+        // (a warp that holds both phases, in a round that is not elastic, runs
+        // them in turn)
+        const bool wssa = __any_sync(FULL, mine_ssa) != 0, wdec = __any_sync(FULL, mine_dec) != 0;
         const uint32_t cap = 8u * run.ssa_budget;  // a round's longest SSA stretch
-        const bool first = lane == (uint32_t)(__ffs(mine_ssa ? smask : dmask) - 1);
-        if (mine_ssa) {
-            bool told = false;
-            for (uint32_t b = 0; b < cap; b++) {
-                if (b == run.ssa_budget && first && !told) {
-                    atomicAdd((uint32_t*)&fin[0], 1u);
-                    told = true;
-                }
-                const bool more = b < run.ssa_budget || (elastic && fin[1] < ndw);
-                const bool act = res == CONT && st.in_ssa && more;
-                if (!__any_sync(smask, act)) break;
-                if (act) res = ssa_step<N, P, SM>(net, run, s, st, o);
-            }
-            if (first && !told) atomicAdd((uint32_t*)&fin[0], 1u);
-        } else if (mine_dec) {
+        int res = CONT;
+        if (wdec) {
             for (uint32_t b = 0; b < run.dec_budget; b++) {
-                const bool act = res == CONT && !st.in_ssa;
-                if (!__any_sync(dmask, act)) break;
-                if (act) res = decide_step<N, P, SM>(net, run, s, st, o);
+                const bool act = mine_dec && res == CONT && !st.in_ssa;
+                if (!__any_sync(FULL, act)) break;
+                const int x = decide_step<N, P, SM>(net, run, w, s, st, o, act);
+                res = act ? x : res;
             }
-            if (first) atomicAdd((uint32_t*)&fin[1], 1u);
-            for (uint32_t b = 0; b < cap && elastic; b++) {
-                const bool act = res == CONT && st.in_ssa && fin[0] < nsw;
-                if (!__any_sync(dmask, act)) break;
-                if (act) res = ssa_step<N, P, SM>(net, run, s, st, o);
-            }
+            if (lane == 0 && elastic) atomicAdd((uint32_t*)&fin[1], 1u);
+        }
+        if (wssa || (wdec && elastic)) {
+            bool told = !wssa;
+            const int x = ssa_steps<N, P, SM>(net, run, w, s, st, o, live && res == CONT && st.in_ssa && (mine_ssa || elastic),
+                                              [&](uint32_t b) {
+                                                  if (!wssa) return b < cap && fin[0] < nsw;
+                                                  if (b < run.ssa_budget) return true;
+                                                  if (!told && lane == 0) atomicAdd((uint32_t*)&fin[0], 1u);
+                                                  told = true;
+                                                  return elastic && b < cap && fin[1] < ndw;
+                                              });
+            res = x == DONE ? x : res;
+            if (!told && lane == 0) atomicAdd((uint32_t*)&fin[0], 1u);
         }
         if (live && res == DONE) {
             finish<N>(net, run, st, o);
@@ -838,12 +981,9 @@ __device__ __forceinline__ void sweep_rounds(const N& net, const dev::Run& run, 
 // simulations per block of the second.
 template <class N, int P, int SM>
 __device__ __forceinline__ void run_sweep(const N& net, const dev::Run& run, uint32_t lanes) {
-    if (run.warp_local) {
-        sweep<N, P, SM>(net, run, lanes);
-    } else {
-        extern __shared__ uint32_t ctl_tiny_xs[];
-        sweep_rounds<N, P, SM>(net, run, lanes, ctl_tiny_xs);
-    }
+    extern __shared__ __align__(16) uint32_t ctl_tiny_xs[];
+    if (run.warp_local) sweep<N, P, SM>(net, run, lanes, ctl_tiny_xs);
+    else sweep_rounds<N, P, SM>(net, run, lanes, ctl_tiny_xs);
 }
 
 }  // namespace tiny

@@ -101,10 +101,11 @@ typedef struct {
     int32_t threads;      /* threads per block; 0 = autotune                           */
     int32_t uniform_rates;/* 1: every row of c equals row 0 (one shared copy per block);
                              ctl_run detects this itself, device calls take it as given */
-    int32_t ssa_budget;   /* SSA steps per simulation and stretch of work (0 = 100; 16 for
-                             the register-resident sweep)                             */
+    int32_t ssa_budget;   /* SSA steps per simulation and stretch of work (0 = 100; 64 or,
+                             with sched 2, 16 for the register-resident sweep)        */
     int32_t dec_budget;   /* leap decisions per simulation and stretch (0 = 2; 8 for
-                             groups of 32 lanes or more)                              */
+                             groups of 32 lanes or more; 4 or, with sched 2, 1 for the
+                             register-resident sweep)                                 */
     int32_t min_blocks;   /* register budget: kernel variant compiled for this many resident
                              256-thread blocks per SM (2: up to 128 registers per thread,
                              3: 80, 4: 64); 0 = library choice (autotuned, else 3 for
@@ -115,7 +116,8 @@ typedef struct {
     int32_t sched;        /* scheduling: 1 = a block's simulations regrouped by phase (warps
                              take them from a pool in shared memory; the register-resident
                              sweep regroups in block rounds), 2 = warp-local (every warp
-                             keeps its own simulations); 0 = library choice.  Groups of 32
+                             keeps its own simulations); 0 = library choice (the register-
+                             resident sweep: by the size of the batch).  Groups of 32
                              lanes or more keep their simulation under either         */
     int32_t warp_sims;    /* register-resident sweep for tiny networks (at most 16 reactions,
                              8 species and sampled species, 3 reactant entries per reaction),
