@@ -15,7 +15,7 @@
 //
 // One B200, batch 16,384, 32 species: a step of forward, backward and Adam took
 // 874 us as 40 launches (a GEMM per product with transposes written 2 bytes at
-// a time, a serial column sum of 108 us per layer, Adam per tensor); here 143
+// a time, a serial column sum of 108 us per layer, Adam per tensor); here 140
 // us as 7.  Bound: the 280 MB that pre-activations, activations and gradients
 // make between the kernels (43 us at the copy rate; 140 MB live, a little more
 // than L2), then the chain of a tile's five layers.
@@ -149,19 +149,21 @@ __device__ __forceinline__ void tr_produce(TrShared& sh, uint8_t* stage, const u
         const uint32_t bytes = (uint32_t)(N(l) * SC_BK * 2);
         for (int ks = 0; ks < K(l) / SC_BK; ks++, idx++) {
             const uint32_t sl = idx % TR_STAGES, round = idx / TR_STAGES;
-            if (round > 0 && !mbar_wait(&sh.empty[sl], (round - 1) & 1u, err)) { ok = false; break; }
-            if (*(volatile int*)&sh.abort) { ok = false; break; }
-            mbar_expect_tx(&sh.full[sl], bytes);
-            bulk_g2s(stage + sl * SC_STAGE_BYTES, w + off, bytes, &sh.full[sl]);
+            if (round > 0 && !mbar_wait_u(&sh.empty[sl], (round - 1) & 1u, err)) { ok = false; break; }
+            if (raised(&sh.abort)) { ok = false; break; }
+            if (elect_one()) {
+                mbar_expect_tx(&sh.full[sl], bytes);
+                bulk_g2s(stage + sl * SC_STAGE_BYTES, w + off, bytes, &sh.full[sl]);
+            }
             issued = idx + 1;
             off += bytes;
         }
     }
     if (!ok) {
-        atomicExch(&sh.abort, 1);
+        if (elect_one()) atomicExch(&sh.abort, 1);
         // let the copies in flight land before the CTA exits
         for (uint32_t i = issued > TR_STAGES ? issued - TR_STAGES : 0u; i < issued; i++)
-            mbar_wait(&sh.full[i % TR_STAGES], (i / TR_STAGES) & 1u, nullptr);
+            mbar_wait_u(&sh.full[i % TR_STAGES], (i / TR_STAGES) & 1u, nullptr);
     }
 }
 
@@ -171,29 +173,29 @@ __device__ __forceinline__ void tr_mma(TrShared& sh, uint32_t stage, uint32_t a,
     uint32_t idx = 0;
     bool ok = true;
     for (int l = 0; l < products && ok; l++) {
-        if (!mbar_wait(&sh.ready, (uint32_t)l & 1u, err) || *(volatile int*)&sh.abort) { ok = false; break; }
+        if (!mbar_wait_u(&sh.ready, (uint32_t)l & 1u, err) || raised(&sh.abort)) { ok = false; break; }
         tc_fence_after();
         const int n = N(l);
         const uint32_t idesc = make_idesc(128, n);
+        const uint32_t kstep = (uint32_t)(2 * (n / 8) * 128), lbo = (uint32_t)((n / 8) * 128);
         for (int ks = 0; ks < K(l) / SC_BK; ks++, idx++) {
             const uint32_t sl = idx % TR_STAGES, round = idx / TR_STAGES;
-            if (!mbar_wait(&sh.full[sl], round & 1u, err)) { ok = false; break; }
+            if (!mbar_wait_u(&sh.full[sl], round & 1u, err)) { ok = false; break; }
             tc_fence_after();
+            if (elect_one()) {
 #pragma unroll
-            for (int kk = 0; kk < SC_BK / 16; kk++) {
-                const uint32_t ka = (uint32_t)((ks * SC_BK + kk * 16) / 8) * 16u * 128u;
-                mma_bf16(tmem, make_desc(a + ka, 16u * 128u, 128u),
-                         make_desc(stage + sl * SC_STAGE_BYTES + (uint32_t)(kk * 2 * (n / 8) * 128),
-                                   (uint32_t)((n / 8) * 128), 128u),
-                         idesc, (ks > 0 || kk > 0) ? 1u : 0u);
+                for (int kk = 0; kk < SC_BK / 16; kk++)
+                    mma_bf16(tmem, make_desc(a + (uint32_t)(ks * 4 + kk * 2) * 16u * 128u, 16u * 128u, 128u),
+                             make_desc(stage + sl * SC_STAGE_BYTES + (uint32_t)kk * kstep, lbo, 128u), idesc,
+                             (ks > 0 || kk > 0) ? 1u : 0u);
+                mma_commit(&sh.empty[sl]);
             }
-            mma_commit(&sh.empty[sl]);
         }
-        if (ok) mma_commit(&sh.acc);
+        if (ok && elect_one()) mma_commit(&sh.acc);
     }
-    if (!ok) atomicExch(&sh.abort, 1);
-    mma_commit(&sh.drain);  // every MMA this thread issued has completed once drain flips
-    mbar_wait(&sh.drain, 0u, nullptr);
+    if (!ok && elect_one()) atomicExch(&sh.abort, 1);
+    if (elect_one()) mma_commit(&sh.drain);  // every MMA this warp issued has completed once drain flips
+    mbar_wait_u(&sh.drain, 0u, nullptr);
 }
 
 __device__ __forceinline__ void tr_finish(uint32_t tmem, int warp) {
@@ -213,7 +215,7 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_forward_kernel(const __gr
     uint8_t* A = smem;
     uint8_t* stage = smem + TR_A_BYTES;
     float* c_bias = reinterpret_cast<float*>(stage + TR_STAGES * SC_STAGE_BYTES);
-    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const int warp = warp_index(), lane = threadIdx.x % 32;
     for (int i = threadIdx.x; i < 4 * SC_HID + p.out_w; i += TR_THREADS)
         c_bias[i] = p.bias[i / SC_HID < 4 ? i / SC_HID : 4][i < 4 * SC_HID ? i % SC_HID : i - 4 * SC_HID];
     tr_init(sh, warp);
@@ -222,9 +224,9 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_forward_kernel(const __gr
     auto N = [&](int l) { return l == TR_L - 1 ? out_w : SC_HID; };
     auto K = [](int l) { return l == 0 ? IN_W : SC_HID; };
     if (warp == 8) {
-        if (lane == 0) tr_produce(sh, stage, p.wpack, TR_L, N, K, p.err);
+        tr_produce(sh, stage, p.wpack, TR_L, N, K, p.err);
     } else if (warp == 9) {
-        if (lane == 0) tr_mma(sh, smem_u32(stage), smem_u32(A), tmem, TR_L, N, K, p.err);
+        tr_mma(sh, smem_u32(stage), smem_u32(A), tmem, TR_L, N, K, p.err);
     } else {
         const int q = warp & 3, h = warp >> 2, r = q * 32 + lane;
         const size_t row = (size_t)blockIdx.x * 128 + r;
@@ -304,16 +306,16 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_backward_kernel(const __g
     __shared__ __align__(8) TrShared sh;
     uint8_t* A = smem;
     uint8_t* stage = smem + TR_A_BYTES;
-    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const int warp = warp_index(), lane = threadIdx.x % 32;
     tr_init(sh, warp);
     const uint32_t tmem = sh.tmem;
     const int out_w = p.out_w;
     auto N = [](int) { return SC_HID; };
     auto K = [&](int i) { return i == 0 ? out_w : SC_HID; };
     if (warp == 8) {
-        if (lane == 0) tr_produce(sh, stage, p.wtpack, 4, N, K, p.err);
+        tr_produce(sh, stage, p.wtpack, 4, N, K, p.err);
     } else if (warp == 9) {
-        if (lane == 0) tr_mma(sh, smem_u32(stage), smem_u32(A), tmem, 4, N, K, p.err);
+        tr_mma(sh, smem_u32(stage), smem_u32(A), tmem, 4, N, K, p.err);
     } else {
         const int q = warp & 3, h = warp >> 2, r = q * 32 + lane;
         const size_t row = (size_t)blockIdx.x * 128 + r;
@@ -413,7 +415,7 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_wgrad_kernel(const __grid
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t full[WG_STAGES], empty[WG_STAGES], done;
     __shared__ uint32_t tmem_slot;
-    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const int warp = warp_index(), lane = threadIdx.x % 32;
     int l = 0;
     while ((int)blockIdx.x >= plan.first[l + 1]) l++;
     const int part = (int)blockIdx.x - plan.first[l], parts = plan.first[l + 1] - plan.first[l];
@@ -444,32 +446,32 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_wgrad_kernel(const __grid
     const uint32_t tmem = tmem_slot;
     bool ok = true;
     if (warp == 8) {
-        if (lane == 0) {
-            int issued = 0;
-            for (int i = 0; i < steps && ok; i++) {
-                const int s = i % WG_STAGES, round = i / WG_STAGES;
-                if (round > 0) ok = mbar_wait(&empty[s], (uint32_t)(round - 1) & 1u, p.err);
-                if (!ok) break;
-                uint8_t* dst = smem + (size_t)s * WG_STAGE_BYTES;
-                const size_t tile = (size_t)(t0 + i / 4), sub = (size_t)(i & 3);
+        int issued = 0;
+        for (int i = 0; i < steps && ok; i++) {
+            const int s = i % WG_STAGES, round = i / WG_STAGES;
+            if (round > 0) ok = mbar_wait_u(&empty[s], (uint32_t)(round - 1) & 1u, p.err);
+            if (!ok) break;
+            uint8_t* dst = smem + (size_t)s * WG_STAGE_BYTES;
+            const size_t tile = (size_t)(t0 + i / 4), sub = (size_t)(i & 3);
+            if (elect_one()) {
                 mbar_expect_tx(&full[s], abytes + bbytes);
                 bulk_g2s(dst, p.dp[l] + tile * 4 * abytes + sub * abytes, abytes, &full[s]);
                 bulk_g2s(dst + WG_STAGE_BYTES / 2, p.hp[l] + tile * 4 * bbytes + sub * bbytes, bbytes, &full[s]);
-                issued = i + 1;
             }
-            if (!ok)  // the copies in flight land before the CTA exits
-                for (int i = issued > WG_STAGES ? issued - WG_STAGES : 0; i < issued; i++)
-                    mbar_wait(&full[i % WG_STAGES], (uint32_t)(i / WG_STAGES) & 1u, nullptr);
+            issued = i + 1;
         }
+        if (!ok)  // the copies in flight land before the CTA exits
+            for (int i = issued > WG_STAGES ? issued - WG_STAGES : 0; i < issued; i++)
+                mbar_wait_u(&full[i % WG_STAGES], (uint32_t)(i / WG_STAGES) & 1u, nullptr);
     } else if (warp == 9) {
-        if (lane == 0) {
-            const uint32_t idesc = make_idesc(128, N);
-            for (int i = 0; i < steps && ok; i++) {
-                const int s = i % WG_STAGES, round = i / WG_STAGES;
-                ok = mbar_wait(&full[s], (uint32_t)round & 1u, p.err);
-                if (!ok) break;
-                tc_fence_after();
-                const uint32_t a = smem_u32(smem + (size_t)s * WG_STAGE_BYTES), b = a + WG_STAGE_BYTES / 2;
+        const uint32_t idesc = make_idesc(128, N);
+        for (int i = 0; i < steps && ok; i++) {
+            const int s = i % WG_STAGES, round = i / WG_STAGES;
+            ok = mbar_wait_u(&full[s], (uint32_t)round & 1u, p.err);
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t a = smem_u32(smem + (size_t)s * WG_STAGE_BYTES), b = a + WG_STAGE_BYTES / 2;
+            if (elect_one()) {
 #pragma unroll
                 for (int kk = 0; kk < 2; kk++) {
                     const uint64_t db = make_desc(b + (uint32_t)(kk * 2 * (N / 8) * 128), (uint32_t)((N / 8) * 128), 128u);
@@ -481,8 +483,8 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_wgrad_kernel(const __grid
                 }
                 mma_commit(&empty[s]);
             }
-            mma_commit(&done);
         }
+        if (elect_one()) mma_commit(&done);
     }
     // (on a timeout the products are not used; the MMAs issued still end first)
     ok = mbar_wait(&done, 0u, p.err) && ok;

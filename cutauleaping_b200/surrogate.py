@@ -165,7 +165,7 @@ class MLP:
     # -- buffers ---------------------------------------------------------------
     def _buf(self, name, shape, dtype):
         t = self._bufs.get(name)
-        if t is None or tuple(t.shape) != tuple(shape) or t.dtype != dtype:
+        if t is None or t.shape != shape or t.dtype != dtype:
             t = self.torch.empty(shape, dtype=dtype, device="cuda")
             self._bufs[name] = t
         return t
@@ -179,23 +179,29 @@ class MLP:
         assert X.shape[1] == IN_PAD
         X = X.contiguous()
         Bn = X.shape[0]
-        self.z = [self._buf(f"z{l}", (Bn, HIDDEN), torch.float32) for l in range(LAYERS)]
-        self.hp = [self._buf(f"hp{l}", (Bn, IN_PAD if l == 0 else HIDDEN), torch.bfloat16)
-                   for l in range(LAYERS + 1)] if keep else None
+        self.z = self._buf("z", (LAYERS, Bn, HIDDEN), torch.float32)
+        self.hp = self._buf("hp", (Bn * (IN_PAD + LAYERS * HIDDEN),), torch.bfloat16) if keep else None
         y = self._buf("y", (Bn, self.out_w), torch.float32)
         d = StepDesc()
         d.X, d.y, d.wpack, d.err = X.data_ptr(), y.data_ptr(), self._wstage().data_ptr(), self.err.data_ptr()
-        for l in range(LAYERS + 1):
-            d.W[l], d.bias[l] = self.Wb[l].data_ptr(), self.b[l].data_ptr()
-            if l < LAYERS:
-                d.z[l] = self.z[l].data_ptr()
-            if keep:
-                d.hp[l] = self.hp[l].data_ptr()
+        d.W[:], d.bias[:] = [w.data_ptr() for w in self.Wb], [v.data_ptr() for v in self.b]
+        d.z[:] = self._z_ptrs(Bn)
+        if keep:
+            d.hp[:] = self._hp_ptrs(Bn)
         d.B, d.out_w = Bn, self.out_w
         st = L.ctl_mlp_forward(C.byref(d), _stream())
         if st != OK:
             raise CtlError(st, "ctl_mlp_forward")
         return y
+
+    # where each layer's part lies in the buffers: FP32 pre-activations, packed layer inputs
+    def _z_ptrs(self, Bn):
+        z = self.z.data_ptr()
+        return [z + l * Bn * HIDDEN * 4 for l in range(LAYERS)]
+
+    def _hp_ptrs(self, Bn):
+        h = self.hp.data_ptr()
+        return [h] + [h + Bn * (IN_PAD + l * HIDDEN) * 2 for l in range(LAYERS)]
 
     def _wstage(self):
         L = _bind()
@@ -207,6 +213,8 @@ class MLP:
         torch = self.torch
         L = _bind()
         Bn, S = target.shape
+        if Bn != self.z.shape[1]:
+            raise ValueError("backward: another batch size than the last forward's")
         y, target = y.contiguous(), target.contiguous()
         # loss and gradients in one zeroed allocation (they are accumulated)
         sizes = [w.numel() for w in self.W] + [b.numel() for b in self.b] + [1]
@@ -215,12 +223,10 @@ class MLP:
         db, loss = list(parts[len(dW):-1]), parts[-1]
         d = StepDesc()
         d.y, d.target, d.loss, d.wpack = y.data_ptr(), target.data_ptr(), loss.data_ptr(), self._wstage().data_ptr()
-        for l in range(LAYERS + 1):
-            d.WT[l], d.hp[l] = self.WbT[l].data_ptr(), self.hp[l].data_ptr()
-            d.dp[l] = self._buf(f"dp{l}", (Bn, 128 if l == LAYERS else HIDDEN), torch.bfloat16).data_ptr()
-            d.dW[l], d.db[l] = dW[l].data_ptr(), db[l].data_ptr()
-            if l < LAYERS:
-                d.z[l] = self.z[l].data_ptr()
+        d.WT[:], d.hp[:], d.z[:] = [w.data_ptr() for w in self.WbT], self._hp_ptrs(Bn), self._z_ptrs(Bn)
+        dp = self._buf("dp", (Bn * (LAYERS * HIDDEN + 128),), torch.bfloat16).data_ptr()
+        d.dp[:] = [dp + l * Bn * HIDDEN * 2 for l in range(LAYERS + 1)]
+        d.dW[:], d.db[:] = [g.data_ptr() for g in dW], [g.data_ptr() for g in db]
         d.B, d.S, d.out_w, d.err = Bn, S, self.out_w, self.err.data_ptr()
         st = L.ctl_mlp_backward(C.byref(d), _stream())
         if st != OK:
@@ -234,9 +240,7 @@ class MLP:
         d = AdamDesc()
         for k, ts in (("w", self.W), ("b", self.b), ("g", dW), ("gb", db), ("m", self.m), ("v", self.v),
                       ("mb", self.mb), ("vb", self.vb), ("wb", self.Wb), ("wbT", self.WbT)):
-            arr = getattr(d, k)
-            for l, t in enumerate(ts):
-                arr[l] = t.data_ptr()
+            getattr(d, k)[:] = [t.data_ptr() for t in ts]
         d.out_w, d.step = self.out_w, self.step_count
         d.lr, d.beta1, d.beta2, d.eps, d.weight_decay = lr, beta1, beta2, eps, wd
         st = L.ctl_mlp_adam_step(C.byref(d), _stream())
