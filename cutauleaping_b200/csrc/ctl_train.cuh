@@ -402,8 +402,12 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_backward_kernel(const __g
 // contraction.  A CTA takes a share of one layer's 128-row tiles and holds the
 // whole [256][K] product in TMEM (two M = 128 halves); per stage it copies 32
 // batch rows of both packed operands.  Shares are sized by the layers' MMAs
-// (layer 0 has K = 64, the last one half the rows).  The sums meet in L2 by
-// vector reductions.
+// (layer 0 has K = 64, the last one half the rows).  A chain of MMA
+// accumulations rounds towards zero at each step, so a share's tiles are cut
+// into as many chains as accumulators fit into TMEM (four of layer 0, two of
+// the last), which the epilogue adds up: no chain is longer than 512 rows up
+// to a batch of 32,768.  The sums meet in L2 by vector reductions.
+__host__ __device__ constexpr int wg_chains(int l) { return l == 0 ? 4 : l == TR_L - 1 ? 2 : 1; }
 constexpr int WG_STAGES = 6;
 constexpr int WG_STAGE_BYTES = 2 * 32 * SC_HID * 2;
 constexpr int WG_SMEM = WG_STAGES * WG_STAGE_BYTES;
@@ -426,7 +430,8 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_wgrad_kernel(const __grid
     const int N = l == 0 ? IN_W : SC_HID;            // columns of dW
     const int halves = arows / 128;
     const uint32_t abytes = (uint32_t)(32 * arows * 2), bbytes = (uint32_t)(32 * N * 2);
-    const int steps = (t1 - t0) * 4;
+    const int steps = (t1 - t0) * 4, chains = min(wg_chains(l), t1 - t0);
+    const uint32_t acols = l == 0 ? IN_W : SC_HID;   // TMEM columns between a half's accumulators
     if (threadIdx.x == 0) {
         for (int i = 0; i < WG_STAGES; i++) {
             mbar_init(&full[i], 1);
@@ -465,8 +470,11 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_wgrad_kernel(const __grid
                 mbar_wait_u(&full[i % WG_STAGES], (uint32_t)(i / WG_STAGES) & 1u, nullptr);
     } else if (warp == 9) {
         const uint32_t idesc = make_idesc(128, N);
+        int chain = -1;
         for (int i = 0; i < steps && ok; i++) {
-            const int s = i % WG_STAGES, round = i / WG_STAGES;
+            const int s = i % WG_STAGES, round = i / WG_STAGES, c = i / 4 * chains / (t1 - t0);
+            const bool add = c == chain;  // else the chain's first product
+            chain = c;
             ok = mbar_wait_u(&full[s], (uint32_t)round & 1u, p.err);
             if (!ok) break;
             tc_fence_after();
@@ -476,10 +484,10 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_wgrad_kernel(const __grid
                 for (int kk = 0; kk < 2; kk++) {
                     const uint64_t db = make_desc(b + (uint32_t)(kk * 2 * (N / 8) * 128), (uint32_t)((N / 8) * 128), 128u);
                     for (int m = 0; m < halves; m++)
-                        mma_bf16(tmem + (uint32_t)(m * SC_HID),
+                        mma_bf16(tmem + (uint32_t)(m * SC_HID) + (uint32_t)c * acols,
                                  make_desc(a + (uint32_t)(kk * 2 * (arows / 8) * 128 + m * 16 * 128),
                                            (uint32_t)((arows / 8) * 128), 128u),
-                                 db, idesc, (i > 0 || kk > 0) ? 1u : 0u);
+                                 db, idesc, (add || kk > 0) ? 1u : 0u);
                 }
                 mma_commit(&empty[s]);
             }
@@ -496,7 +504,14 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_wgrad_kernel(const __grid
             const int n = m * 128 + q * 32 + lane;  // row of dW
             for (int c = (warp >> 2) * 32; c < N; c += 64) {
                 float v[32];
-                tmem_ld32(tmem + (uint32_t)(m * SC_HID) + ((uint32_t)(q * 32) << 16) + (uint32_t)c, v);
+                const uint32_t at = tmem + (uint32_t)(m * SC_HID) + ((uint32_t)(q * 32) << 16) + (uint32_t)c;
+                tmem_ld32(at, v);
+                for (int a = 1; a < chains; a++) {
+                    float u[32];
+                    tmem_ld32(at + (uint32_t)a * acols, u);
+#pragma unroll
+                    for (int k = 0; k < 32; k++) v[k] += u[k];
+                }
                 if (n < mrows)
 #pragma unroll
                     for (int k = 0; k < 32; k += 4)
