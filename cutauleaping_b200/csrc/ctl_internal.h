@@ -66,6 +66,14 @@ struct ctl_model {
     // autotune cache: (device, log2 of the batch size, rate mode, flags) -> launch shape
     struct Tuned { int device; uint32_t nbucket, uniform, flags; int group, threads, ssa_budget, dec_budget, min_blocks, sched, warp_sims; };
     std::vector<Tuned> tuned;
+    // kept between calls, under keep_mu: idle streams of ctl_run (device,
+    // cudaStream_t; at most KEEP_STREAMS, destroyed with the model) and the
+    // register-resident kernels compiled for the network
+    static constexpr int KEEP_STREAMS = 4;
+    std::mutex keep_mu;
+    struct Idle { int device; void* stream; } idle[KEEP_STREAMS] = {};  // stream null: free place
+    struct TinySpec { uint32_t flags; int min_blocks, sched; const void* kernel; };
+    std::vector<TinySpec> tiny_spec;
 };
 
 struct ctl_target {

@@ -449,7 +449,20 @@ static int tiny_sched(const ctl_run_cfg* cfg, uint32_t n, int sm_count) {
 // simulations: 538k sims/s with 2, 551k with 1, 555k with none).
 static constexpr uint32_t TINY_TAIL_SIMS = 1;
 
-static ctl_status plan_tiny(const HostTables& t, const ctl_run_cfg* cfg, uint32_t n, LaunchPlan& pl) {
+// tiny_spec_kernel, looked up by what its source depends on (writing the source
+// to look it up takes longer than a small launch).
+static const void* tiny_kernel_of(ctl_model* m, uint32_t flags, int minb, int sched) {
+    flags &= dev::F_Q5_OFF;
+    std::lock_guard<std::mutex> lk(m->keep_mu);
+    for (const auto& e : m->tiny_spec)
+        if (e.flags == flags && e.min_blocks == minb && e.sched == sched) return e.kernel;
+    const void* k = tiny_spec_kernel(m->t, flags, minb, sched, nullptr);
+    m->tiny_spec.push_back({flags, minb, sched, k});
+    return k;
+}
+
+static ctl_status plan_tiny(ctl_model* m, const ctl_run_cfg* cfg, uint32_t n, LaunchPlan& pl) {
+    const HostTables& t = m->t;
     DevAttr da;
     if (device_attr(cfg->device, da) != CTL_OK) return CTL_ERR_CUDA;
     pl.tinyP = t.P;
@@ -461,7 +474,7 @@ static ctl_status plan_tiny(const HostTables& t, const ctl_run_cfg* cfg, uint32_
     // against 295k sims/s; 65,536: 722k against 650k
     const int minb = cfg->min_blocks > 0 ? cfg->min_blocks : 1;
     const int sched = cfg->sched > 0 ? cfg->sched : tiny_sched(cfg, n, da.sm_count);
-    pl.spec = cfg->spec >= 0 ? tiny_spec_kernel(t, cfg->flags, minb, sched, nullptr) : nullptr;
+    pl.spec = cfg->spec >= 0 ? tiny_kernel_of(m, cfg->flags, minb, sched) : nullptr;
     const void* k = pl.spec ? pl.spec : tiny_kernel_ptr(pl.tinyP, pl.tinySM);
     if (!k) {
         set_error("no register-resident kernel for this network");
@@ -594,7 +607,7 @@ static ctl_status plan_launch(ctl_model* m, const ctl_run_cfg* cfg_in, uint32_t 
         return CTL_ERR_ARG;
     }
     if (tiny_ok && (cfg->warp_sims > 0 || (cfg->warp_sims == 0 && cfg->group <= 0)))
-        return plan_tiny(t, cfg, n, pl);
+        return plan_tiny(m, cfg, n, pl);
     if (cfg->min_blocks == 1) {
         set_error("min_blocks 1 applies to the register-resident sweep only; the shared-memory sweep takes 2, 3 or 4");
         return CTL_ERR_ARG;
@@ -848,6 +861,8 @@ struct ctl_graph {
 
 extern "C" void ctl_model_free(ctl_model* m) {
     if (!m) return;
+    for (const auto& i : m->idle)
+        if (i.stream) cudaStreamDestroy(static_cast<cudaStream_t>(i.stream));
     for (auto& d : m->dev) {
         if (d.buf) {
             int prev = 0;
@@ -906,6 +921,35 @@ extern "C" ctl_status ctl_run_device(ctl_model* m, const ctl_run_cfg* cfg, uint3
     return enqueue_sweep(m, cfg, n, d_X0, d_c, d_samples, d_info, static_cast<cudaStream_t>(stream), pl, *d);
 }
 
+// A non-blocking stream of the current device for one call, kept by the model
+// between calls: creating and destroying one takes 0.11 ms, and a call on 64
+// Schlogl simulations, which takes 0.9 ms on the device, used two.
+static cudaError_t take_stream(ctl_model* m, int device, cudaStream_t& s) {
+    {
+        std::lock_guard<std::mutex> lk(m->keep_mu);
+        for (auto& i : m->idle)
+            if (i.stream && i.device == device) {
+                s = static_cast<cudaStream_t>(i.stream);
+                i.stream = nullptr;
+                return cudaSuccess;
+            }
+    }
+    return cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+}
+
+// `done`: all work on it has completed without an error.
+static void give_stream(ctl_model* m, int device, cudaStream_t s, bool done) {
+    if (done) {
+        std::lock_guard<std::mutex> lk(m->keep_mu);
+        for (auto& i : m->idle)
+            if (!i.stream) {
+                i = {device, s};
+                return;
+            }
+    }
+    cudaStreamDestroy(s);
+}
+
 extern "C" ctl_status ctl_run(ctl_model* m, const ctl_run_cfg* cfg, uint32_t n, const int32_t* X0,
                               const float* c, uint32_t* samples, ctl_sim_info* info) {
     if (!m) return CTL_ERR_ARG;
@@ -954,10 +998,10 @@ extern "C" ctl_status ctl_run(ctl_model* m, const ctl_run_cfg* cfg, uint32_t n, 
     while (((uint64_t)n >> shift) > 16) shift++;
     const uint32_t nch = (uint32_t)(((uint64_t)n + (1ull << shift) - 1) >> shift);
     const bool overlap = !out_host && bo >= ((size_t)64 << 20) && nch > 1;
-    cudaStream_t s, cs;
-    CTL_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    if (cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking) != cudaSuccess) {
-        cudaStreamDestroy(s);
+    cudaStream_t s = nullptr, cs = nullptr;
+    CTL_CUDA(take_stream(m, cfg->device, s));
+    if (overlap && take_stream(m, cfg->device, cs) != cudaSuccess) {
+        give_stream(m, cfg->device, s, true);
         return cuda_fail(cudaErrorMemoryAllocation, "ctl_run (copy stream)");
     }
     void *dx = nullptr, *dc = nullptr, *dout = nullptr, *dinf = nullptr, *ddone = nullptr;
@@ -1015,7 +1059,7 @@ extern "C" ctl_status ctl_run(ctl_model* m, const ctl_run_cfg* cfg, uint32_t n, 
                                 cudaMemcpyDeviceToHost, s);
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(info, dinf, bi, cudaMemcpyDeviceToHost, s);
-    const cudaError_t e3 = cudaStreamSynchronize(cs);  // copies in flight end before the buffers go
+    const cudaError_t e3 = cs ? cudaStreamSynchronize(cs) : cudaSuccess;  // copies in flight end before the buffers go
     if (dx) cudaFreeAsync(dx, s);
     if (dc) cudaFreeAsync(dc, s);
     if (dout) cudaFreeAsync(dout, s);
@@ -1023,8 +1067,9 @@ extern "C" ctl_status ctl_run(ctl_model* m, const ctl_run_cfg* cfg, uint32_t n, 
     if (ddone) cudaFreeAsync(ddone, s);
     const cudaError_t e2 = cudaStreamSynchronize(s);
     if (hdone) cudaFreeHost(hdone);
-    cudaStreamDestroy(cs);
-    cudaStreamDestroy(s);
+    const bool done = e == cudaSuccess && e2 == cudaSuccess && e3 == cudaSuccess;
+    if (cs) give_stream(m, cfg->device, cs, done);
+    give_stream(m, cfg->device, s, done);
     if (st != CTL_OK) return st;
     if (e != cudaSuccess) return cuda_fail(e, "ctl_run");
     if (e3 != cudaSuccess) return cuda_fail(e3, "ctl_run (copies)");
