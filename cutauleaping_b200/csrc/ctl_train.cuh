@@ -15,10 +15,12 @@
 //
 // One B200, batch 16,384, 32 species: a step of forward, backward and Adam took
 // 874 us as 40 launches (a GEMM per product with transposes written 2 bytes at
-// a time, a serial column sum of 108 us per layer, Adam per tensor); here 140
-// us as 7.  Bound: the 280 MB that pre-activations, activations and gradients
-// make between the kernels (43 us at the copy rate; 140 MB live, a little more
-// than L2), then the chain of a tile's five layers.
+// a time, a serial column sum of 108 us per layer, Adam per tensor); here 124
+// us as 7 (140 before the pre-activations lay in the order of the lanes that
+// store and load them, and y and the target were read by whole lines).  Bound:
+// the 280 MB that pre-activations, activations and gradients make between the
+// kernels (43 us at the copy rate; 140 MB live, a little more than L2), then
+// the chain of a tile's five layers.
 #pragma once
 
 namespace ctl {
@@ -35,7 +37,7 @@ struct Train {
     const uint8_t* wpack;        // forward weights, stages of 32 K-columns
     const uint8_t* wtpack;       // backward weights (W^T of layers 4, 3, 2, 1)
     const float* bias[TR_L];
-    float* z[4];                 // [B][256] pre-activations
+    float* z[4];                 // [B][256] pre-activations, in the order of z_at
     float* y;                    // [B][out_w]
     uint8_t* hp[TR_L];           // packed transposed inputs of each layer: [0] X, [l] the activations of layer l - 1; or null
     uint8_t* dp[TR_L];           // packed transposed gradients of each layer's output ([4]: 128 rows)
@@ -105,6 +107,13 @@ __device__ __forceinline__ void tile_transpose(uint32_t a, int cols, int prows, 
             if ((lane & 3) == 0) atomicAdd(sums + kb * 8 + (lane >> 2), s);
         }
     }
+}
+
+// Where a lane of an epilogue warp keeps its part of a tile's pre-activations:
+// 16 groups of 8 columns of its row, each group next to its neighbour lanes'
+// (a warp's 32-byte stores then fill 8 lines, where rows 1 KB apart touched 32).
+__device__ __forceinline__ size_t z_at(int warp, int lane) {
+    return ((size_t)(blockIdx.x * 8 + warp) * 16 * 32 + lane) * 8;
 }
 
 // Barriers and TMEM of a forward or backward CTA.
@@ -232,9 +241,11 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_forward_kernel(const __gr
         const size_t row = (size_t)blockIdx.x * 128 + r;
         const uint32_t tbase = tmem + ((uint32_t)(q * 32) << 16);
 #pragma unroll
-        for (int kb = 0; kb < 4; kb++)
-            *reinterpret_cast<uint4*>(A + canon(r, (4 * h + kb) * 8, 128)) =
-                *reinterpret_cast<const uint4*>(p.X + row * IN_W + (4 * h + kb) * 8);
+        for (int i = 0; i < 4; i++) {  // eight lanes a row: whole lines
+            const int xr = 32 * i + (int)threadIdx.x / 8, xc = 8 * ((int)threadIdx.x % 8);
+            *reinterpret_cast<uint4*>(A + canon(xr, xc, 128)) =
+                *reinterpret_cast<const uint4*>(p.X + ((size_t)blockIdx.x * 128 + xr) * IN_W + xc);
+        }
         fence_async_smem();
         mbar_arrive_warp(&sh.ready);
         if (p.hp[0]) {
@@ -250,7 +261,8 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_forward_kernel(const __gr
             tc_fence_after();
             const float* b = c_bias + l * SC_HID;
             const int width = N(l), c0 = h * (width / 2), nc = width / 64;  // 32-column chunks of this half
-            float* zout = (l < TR_L - 1 ? p.z[l] : p.y) + row * width;
+            float* zout = l < TR_L - 1 ? p.z[l] + z_at(warp, lane) : p.y + row * width + c0;
+            const int zstep = l < TR_L - 1 ? 256 : 8;
             uint32_t ra[32], rb[32];
             tmem_ld32_issue(tbase + (uint32_t)c0, ra);
 #pragma unroll 1
@@ -270,7 +282,7 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_forward_kernel(const __gr
                         float z[8];
 #pragma unroll
                         for (int e = 0; e < 8; e++) z[e] = __uint_as_float(cur[8 * k + e]) + bias[e];
-                        st8(zout + c + 8 * k, z);
+                        st8(zout + (4 * (j + u) + k) * zstep, z);
                         if (l < TR_L - 1) {
                             uint4 o;
                             o.x = pack_bf2(silu(z[0]), silu(z[1]));
@@ -318,35 +330,31 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_backward_kernel(const __g
         tr_mma(sh, smem_u32(stage), smem_u32(A), tmem, 4, N, K, p.err);
     } else {
         const int q = warp & 3, h = warp >> 2, r = q * 32 + lane;
-        const size_t row = (size_t)blockIdx.x * 128 + r;
         const uint32_t tbase = tmem + ((uint32_t)(q * 32) << 16);
         {
-            // half 0: means, half 1: log-variances; each pair (mu, lv) of a
-            // row is read by both
+            // a warp's lanes take a row's species side by side (whole lines of y
+            // and target; a lane per row touched 32 lines with each load)
             const int S = p.S;
-            const float* y = p.y + row * out_w;
-            const float* tg = p.target + row * S;
             const float sc = 1.0f / ((float)p.B * (float)S);
             float l = 0.0f;
-            auto grad = [&](int s) {  // output column s of this row
-                const bool isv = s >= S;
-                const int k = isv ? s - S : s;
-                if (k >= S) return 0.0f;
-                const float mu = y[k];
-                float lv = y[S + k];
-                lv = fminf(fmaxf(lv, -12.0f), 12.0f);
-                const float iv = __expf(-lv);
-                const float d = tg[k] - mu;
-                if (isv) return 0.5f * (1.0f - d * d * iv) * sc;
-                l += 0.5f * (lv + d * d * iv);
-                return -d * iv * sc;
+            auto put = [&](int rr, int c, float v) {
+                *reinterpret_cast<__nv_bfloat16*>(A + canon(rr, c, 128)) = __float2bfloat16(v);
             };
-            for (int c = h * (out_w / 2); c < (h + 1) * (out_w / 2); c += 8) {
-                float v[8];
-#pragma unroll
-                for (int e = 0; e < 8; e++) v[e] = grad(c + e);
-                *reinterpret_cast<uint4*>(A + canon(r, c, 128)) =
-                    make_uint4(pack_bf2(v[0], v[1]), pack_bf2(v[2], v[3]), pack_bf2(v[4], v[5]), pack_bf2(v[6], v[7]));
+#pragma unroll 4
+            for (int rr = warp; rr < 128; rr += 8) {
+                const float* y = p.y + ((size_t)blockIdx.x * 128 + rr) * out_w;
+                const float* tg = p.target + ((size_t)blockIdx.x * 128 + rr) * S;
+                for (int k = lane; k < S; k += 32) {
+                    const float mu = y[k];
+                    float lv = y[S + k];
+                    lv = fminf(fmaxf(lv, -12.0f), 12.0f);
+                    const float iv = __expf(-lv);
+                    const float d = tg[k] - mu;
+                    l += 0.5f * (lv + d * d * iv);
+                    put(rr, k, -d * iv * sc);
+                    put(rr, S + k, 0.5f * (1.0f - d * d * iv) * sc);
+                }
+                for (int k = 2 * S + lane; k < out_w; k += 32) put(rr, k, 0.0f);
             }
             for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
             if (lane == 0 && l != 0.0f) atomicAdd(p.loss, l);
@@ -357,6 +365,10 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_backward_kernel(const __g
         tile_transpose(smem_u32(A), out_w, 128, p.dp[4] + (size_t)blockIdx.x * 128 * 128 * 2, p.db[4], warp, lane);
         for (int i = 0; i < 4; i++) {
             const int l = 3 - i;
+            const float* zin = p.z[l] + z_at(warp, lane);
+            float z[2][4][8];  // a chunk's pre-activations, loaded a chunk ahead
+#pragma unroll
+            for (int k = 0; k < 4; k++) ld8(zin + k * 256, z[0][k]);
             bool got = mbar_wait(&sh.acc, (uint32_t)i & 1u, p.err);
             if (!tr_all(got && !*(volatile int*)&sh.abort)) {
                 atomicExch(&sh.abort, 1);
@@ -364,7 +376,6 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_backward_kernel(const __g
             }
             tc_fence_after();
             const int c0 = 128 * h;
-            const float* zin = p.z[l] + row * SC_HID;
             uint32_t ra[32], rb[32];
             tmem_ld32_issue(tbase + (uint32_t)c0, ra);
 #pragma unroll 1
@@ -372,9 +383,9 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_backward_kernel(const __g
 #pragma unroll
                 for (int u = 0; u < 2; u++) {
                     const int c = c0 + 32 * (j + u);
-                    float z[4][8];
+                    if (j + u + 1 < 4)
 #pragma unroll
-                    for (int k = 0; k < 4; k++) ld8(zin + c + 8 * k, z[k]);
+                        for (int k = 0; k < 4; k++) ld8(zin + (4 * (j + u + 1) + k) * 256, z[u ^ 1][k]);
                     tmem_wait();
                     uint32_t(&cur)[32] = u ? rb : ra;
                     if (j + u + 1 < 4) tmem_ld32_issue(tbase + (uint32_t)(c + 32), u ? ra : rb);
@@ -382,7 +393,7 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_backward_kernel(const __g
                     for (int k = 0; k < 4; k++) {
                         float d[8];
 #pragma unroll
-                        for (int e = 0; e < 8; e++) d[e] = __uint_as_float(cur[8 * k + e]) * silu_grad(z[k][e]);
+                        for (int e = 0; e < 8; e++) d[e] = __uint_as_float(cur[8 * k + e]) * silu_grad(z[u][k][e]);
                         *reinterpret_cast<uint4*>(A + canon(r, c + 8 * k, 128)) = make_uint4(
                             pack_bf2(d[0], d[1]), pack_bf2(d[2], d[3]), pack_bf2(d[4], d[5]), pack_bf2(d[6], d[7]));
                     }

@@ -374,7 +374,8 @@ typedef struct {
     const void* W[5];       /* forward: BF16 [256][64], [256][256] x 3, [out_w][256] */
     const void* WT[5];      /* backward: their transposes (WT[0] is not read) */
     const float* bias[5];   /* forward: [256] x 4, [out_w] */
-    float* z[4];            /* [B][256] pre-activations: written forward, read backward (32-byte aligned) */
+    float* z[4];            /* B * 256 pre-activations, in an order of the kernels' own: written forward,
+                               read backward (32-byte aligned) */
     float* y;               /* [B][out_w]: written forward, read backward (32-byte aligned) */
     void* hp[5];            /* the layers' inputs in the weight gradients' order, B * 128 bytes, B * 512 x 4: written
                                forward (where not NULL), read backward */
