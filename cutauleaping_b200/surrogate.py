@@ -208,14 +208,25 @@ class MLP:
         return self._buf("wstage", (L.ctl_mlp_pack_bytes(self.out_w) // 2,), self.torch.bfloat16)
 
     def backward(self, y, target):
-        """Gaussian NLL of y = [mu | log var] against target [B][S]; returns
-        (loss sum, gradients dW[l], db[l])."""
+        """Gaussian NLL of y = [mu | log var | ...] (FP32 [B][2S or more], any
+        row stride) against target [B][S] (FP32); returns (loss sum, gradients
+        dW[l], db[l])."""
         torch = self.torch
         L = _bind()
         Bn, S = target.shape
         if Bn != self.z.shape[1]:
             raise ValueError("backward: another batch size than the last forward's")
-        y, target = y.contiguous(), target.contiguous()
+        if y.dim() != 2 or y.shape[0] != Bn or y.shape[1] < 2 * S:
+            raise ValueError("backward: y must be [B][2S] or wider, as forward returns it")
+        if any(t.dtype != torch.float32 or t.device != self.err.device for t in (y, target)):
+            raise ValueError("backward: y and target must be FP32 tensors on the network's device")
+        # the kernel steps y by rows of out_w floats from a 32-byte boundary
+        if y.shape[1] != self.out_w or not y.is_contiguous() or y.data_ptr() % 32:
+            w = min(2 * S, self.out_w)
+            rows = self._buf("y_rows", (Bn, self.out_w), torch.float32)
+            rows[:, :w].copy_(y[:, :w])
+            y = rows
+        target = target.contiguous()
         # loss and gradients in one zeroed allocation (they are accumulated)
         sizes = [w.numel() for w in self.W] + [b.numel() for b in self.b] + [1]
         parts = torch.zeros(sum(sizes), device="cuda").split(sizes)
