@@ -300,6 +300,9 @@ __device__ __forceinline__ float prop(const M& m, const Slot<M>& sl, int r, uint
 // levels (three barriers, 8 loads per node and lane).  The sums are those of
 // the binary tree, level by level.  Lanes with more chunks than registers hold
 // (a group smaller than the library would take) sum them again as they descend.
+// Groups of several warps exchange their totals through the group's scratch:
+// tree_build and descend read them until the next tree_build, which waits for
+// the group before it writes (a leap builds two critical trees in a row).
 template <int G, class M>
 struct Tree {
     // chunks kept in registers
@@ -369,6 +372,7 @@ __device__ __forceinline__ void tree_build(const Grp<G>& g, const M& m, const Sl
         s = s + t.part[j];
     }
     if constexpr (G > 32) {
+        g.sync();  // the totals of the tree before have been read
         if ((g.lane & 31u) == 0) g.ts[g.warp()] = s;
         g.sync();
         if constexpr (G == 64) s = g.ts[0] + g.ts[1];
