@@ -314,18 +314,21 @@ struct Tree {
     double root;
 };
 
-// Chunk q's leaves.  Mode 0: propensities; 1: those of critical reactions
-// (a - am: am is a or 0); 2: as 1 but leaf 0 unmasked (the reference's
-// critical pick, tau.cu:1997).
+// Chunk q's leaves.  Mode 0: propensities; 1: those of critical reactions: am
+// holds a copy of a, or 0 where the reaction is critical, so their exclusive or
+// is 0 or a, whatever a is (a - am would be no number where a propensity
+// overflows FP32); 2: as 1 but leaf 0 unmasked (the reference's critical pick,
+// tau.cu:1997).
 template <class M>
 __device__ __forceinline__ float4 leaves(const M& m, const Slot<M>& sl, int q, int mode) {
     float4 v = sl.chunk(m, q);
     if (mode) {
         const float4 n = reinterpret_cast<const float4*>(sl.am(m))[q];
-        v.x = mode == 2 && q == 0 ? v.x : v.x - n.x;
-        v.y = v.y - n.y;
-        v.z = v.z - n.z;
-        v.w = v.w - n.w;
+        auto critical = [](float a, float am) { return __uint_as_float(__float_as_uint(a) ^ __float_as_uint(am)); };
+        v.x = mode == 2 && q == 0 ? v.x : critical(v.x, n.x);
+        v.y = critical(v.y, n.y);
+        v.z = critical(v.z, n.z);
+        v.w = critical(v.w, n.w);
     }
     return v;
 }
