@@ -1295,17 +1295,9 @@ extern "C" ctl_status ctl_mlp_backward(const ctl_mlp_step_desc* d, void* stream)
     p.err = d->err;
     mlp::train_backward_kernel<<<d->B / 128, mlp::TR_THREADS, mlp::TR_SMEM, s>>>(p);
     if ((st = mlp_cuda(cudaGetLastError(), "train_backward_kernel launch")) != CTL_OK) return st;
-    // CTAs per layer by the layer's MMA time per 128 rows (layer 0: a quarter
-    // of the columns; the last: half the rows), one per SM in all; more where
-    // a batch of more than 16,384 would make the accumulation chains long
-    const double cost[mlp::TR_L] = {0.35, 1.0, 1.0, 1.0, 0.5};
-    const int tiles = d->B / 128;
     mlp::WgPlan plan;
     plan.first[0] = 0;
-    for (int l = 0; l < mlp::TR_L; l++)
-        plan.first[l + 1] = plan.first[l] + std::max(
-            1, std::min(tiles, std::max((int)(sms * cost[l] / 3.85), (std::min(64, d->B / 512) + mlp::wg_chains(l) - 1) /
-                                                                          mlp::wg_chains(l))));
+    for (int l = 0; l < mlp::TR_L; l++) plan.first[l + 1] = plan.first[l] + mlp::wg_ctas(l, d->B / 128, sms);
     mlp::train_wgrad_kernel<<<plan.first[mlp::TR_L], mlp::TR_THREADS, mlp::WG_SMEM, s>>>(p, plan);
     return mlp_cuda(cudaGetLastError(), "train_wgrad_kernel launch");
 }

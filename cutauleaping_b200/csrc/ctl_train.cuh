@@ -23,10 +23,12 @@
 // the chain of a tile's five layers.
 #pragma once
 
+#include "ctl_train_plan.h"
+
 namespace ctl {
 namespace mlp {
 
-constexpr int TR_L = 5, IN_W = 64;                // layers, input width
+constexpr int IN_W = 64;                          // input width
 constexpr int TR_EPI = 256, TR_THREADS = TR_EPI + 64;
 constexpr int TR_STAGES = 5;                      // weight stages of 32 K-columns
 constexpr int TR_A_BYTES = 128 * SC_HID * 2;
@@ -416,9 +418,8 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_backward_kernel(const __g
 // (layer 0 has K = 64, the last one half the rows).  A chain of MMA
 // accumulations rounds towards zero at each step, so a share's tiles are cut
 // into as many chains as accumulators fit into TMEM (four of layer 0, two of
-// the last), which the epilogue adds up: no chain is longer than 512 rows up
-// to a batch of 32,768.  The sums meet in L2 by vector reductions.
-__host__ __device__ constexpr int wg_chains(int l) { return l == 0 ? 4 : l == TR_L - 1 ? 2 : 1; }
+// the last), which the epilogue adds up; ctl_train_plan.h bounds their length.
+// The sums meet in L2 by vector reductions.
 constexpr int WG_STAGES = 6;
 constexpr int WG_STAGE_BYTES = 2 * 32 * SC_HID * 2;
 constexpr int WG_SMEM = WG_STAGES * WG_STAGE_BYTES;
