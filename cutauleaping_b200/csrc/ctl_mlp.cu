@@ -631,11 +631,15 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
 #pragma unroll
     for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
-// One lane waits for its warp.
+// One lane waits for its warp.  The shuffle hands over the answer but orders no
+// memory: the barrier does, between that lane's acquire and the accumulator and
+// shared memory that the other lanes go on to.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, unsigned* err) {
     bool ok = true;
     if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, err);
-    return __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+    ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+    __syncwarp();
+    return ok;
 }
 
 // Byte offset of (row, k) in a K-major no-swizzle tile with `rows` rows.
