@@ -689,6 +689,10 @@ static ctl_status plan_launch(ctl_model* m, const ctl_run_cfg* cfg_in, uint32_t 
     pl.G = G;
     int bps = 0, regs = 0;
     if (ctl_status st = occupancy(dev_id, kern, threads, pl.smem, bps, regs); st != CTL_OK) return st;
+    if (bps < 1) {
+        set_error("sweep kernel cannot be resident with this shape");
+        return CTL_ERR_SHAPE;
+    }
     if (const uint64_t cap = (uint64_t)bps * da.sm_count; G < 32 && pl.sched == 1 && (uint64_t)n > cap * pl.NS) {
         // more slots than groups, as many as the resident blocks' shared
         // memory holds (at most a quarter as many again): simulations that
@@ -712,10 +716,6 @@ static ctl_status plan_launch(ctl_model* m, const ctl_run_cfg* cfg_in, uint32_t 
     if (pl.dec_budget <= 0) pl.dec_budget = default_dec_budget(G);
     pl.threads = threads;
     pl.minb = minb;
-    if (bps < 1) {
-        set_error("sweep kernel cannot be resident with this shape");
-        return CTL_ERR_SHAPE;
-    }
     pl.regs = regs;
     pl.blocks_per_sm = bps;
     pl.sm_count = da.sm_count;
