@@ -623,11 +623,24 @@ static ctl_status plan_launch(ctl_model* m, const ctl_run_cfg* cfg_in, uint32_t 
         if (device_attr(cfg->device, da0) != CTL_OK) return CTL_ERR_CUDA;
         const int gmax = std::min(t.P, 32);
         while (G < gmax && (uint64_t)n * G < (uint64_t)256 * da0.sm_count) G <<= 1;
-        // groups of several warps: half the lanes where that makes one wave of
-        // a batch that would take a little more (three blocks of 256 threads
-        // per SM hold 768 / G simulations)
-        const uint64_t cap = (uint64_t)da0.sm_count * (768 / G);
-        if (G > 32 && n > cap && n <= 2 * cap) G >>= 1;
+        // Groups of several warps that leap: twice the lanes for a batch that two
+        // blocks per SM then hold, and for one that takes up to a quarter more
+        // than a wave of the resident blocks (the second wave is nearly empty).
+        // One B200, ms with 64 and 128 lanes for 512 x 1024 to t 0.02, 128 and
+        // 256 for 1,024 x 2,048 to t 0.01: 64 simulations 67 and 40, 113 and 74;
+        // two blocks per SM (592, 296) 74 and 53, 121 and 87; a quarter more
+        // than a wave (2,200, 1,000) 219 and 202, 414 and 353.  Where the line
+        // leaves the fewer lanes: (1,184, 460) 95 and 128, 147 and 226; (2,664,
+        // 1,400) 227 and 233, 432 and 474.  Exact steps alone, 512 x 1024: 600
+        // simulations 6.2 and 8.7, 2,000 14 and 21.  Half the lanes lose: 3,000
+        // simulations of 512 x 1024 take 254 with 64, 368 with 32.
+        if (G > 32 && G < 256 && !(cfg->flags & dev::F_FORCE_SSA)) {
+            dev::Layout lay;
+            const size_t block = slot_layout(t, G, 256 / G, cfg->uniform_rates != 0, lay, sums) + 1024;
+            const uint64_t blocks = std::min<size_t>(3, ((size_t)da0.smem_optin + 1024) / block);
+            const uint64_t wave = (uint64_t)da0.sm_count * blocks * (256 / G);
+            if ((uint64_t)n * 2 * G <= (uint64_t)512 * da0.sm_count || (n > wave && (uint64_t)4 * n <= 5 * wave)) G <<= 1;
+        }
     }
     if (G != 1 && G != 2 && G != 4 && G != 8 && G != 16 && G != 32 && G != 64 && G != 128 && G != 256) {
         set_error("group must be a power of two from 1 to 256");
