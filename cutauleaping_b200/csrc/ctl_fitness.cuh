@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 #include <cooperative_groups.h>
 
+#include <algorithm>
 #include <cstdint>
 
 namespace ctl {
@@ -236,13 +237,40 @@ struct Shape {
     int cl, loaders;  // CTAs per parameter set (0: one thread per set), loader threads per CTA
 };
 
-// One B200, microseconds measured over 2,048 to 131,072 sets of 60 to 1,600
-// words: a thread per set takes about words * (0.45 + 0.06 p_rep) whatever the
-// number of sets (its serial loads' latency), a CTA of 128 loaders per set
-// sets / SMs * (0.85 + 0.0057 words) (the chains of the CTAs an SM holds).
-// 65,536 sets, 400 words, p_rep 4: 467 against 1,449; 8,192 sets, 400 words,
-// p_rep 8: 355 against 200; from p_rep 32 on the thread's uncoalesced rows
-// thrash the caches (32,768 sets, 60 words: 858 against 347).
+// Microseconds of the two kernels, as measured on one B200 over 64 to 262,144
+// sets of 3 to 1,600 words, 1 to 128 samples (or sums) a word and 1 to 16 target
+// repetitions (13,459 shapes).
+//
+// A thread per set: the latency of its serial loads, whatever the number of
+// sets, then the sectors that the sets load together.  A warp's lanes share
+// sectors where neighbouring sets' rows lie side by side (`threads` of 16 or
+// more, or sums) and are shorter than one; a word's sectors serve the words
+// after it while the rows under way fit an SM's L1, else they come from L2 or
+// HBM again, whole lines apart when a row is longer than one.
+inline double lane_us(const Args& a, int sms) {
+    const double words = (double)a.ns * a.so, sets = a.nsets, rep = a.REP;
+    const double rows = a.samples ? a.p_rep : 1.0;
+    const bool side = !a.samples || a.threads >= 16u;
+    const double share = std::min(1.0, (side ? words : words * rows) / 8.0);  // of a 32-byte sector
+    const bool keeps = std::min(sets / sms, 2048.0) * rows * share * 32.0 <= 200e3;
+    const double sector = keeps ? 1.1e-6 : words <= 32.0 ? 4.0e-6 : 14e-6;
+    return 3.3 + words * (0.26 + (side ? 0.030 : 0.048) * rows + 0.13 * rep) +
+           sets * words * (share * rows * sector + 0.72e-6 * rep);
+}
+
+// A CTA of 128 loaders per set: a launch and one set, or what the sets of an SM
+// cost it -- the chain of their terms above all.
+inline double cta_us(const Args& a, int sms) {
+    const double words = (double)a.ns * a.so, sets = a.nsets, rep = a.REP, rows = a.samples ? a.p_rep : 1.0;
+    return std::max(7.0 + 0.15 * rep + 0.002 * sets,
+                    sets / sms * (1.2 + 0.0005 * rows + 0.06 * rep + words * (0.0051 * rep + 0.000072 * rows)));
+}
+
+// The kernel with the smaller estimate: 0.7 % slower than the faster kernel on
+// the average of those shapes, and at most 2.5 us slower than a thread per set.
+// 65,536 sets of 6 words and 64 samples take 103 us with a thread per set and 400
+// with a CTA; 32,768 of 60 words and 32 samples 915 and 363; 256 of 60 words and
+// one sample 29 and 7.
 // Large sets (from 2^18 samples, 1 MB): 256 sets of 512 x 1,600 samples take
 // 182 on two CTAs of 128 loaders each, 190 on one of 512, 273 on one of 128;
 // 8 such sets take 62, 48 and 102, so fewer sets than half the SMs get 512.
@@ -250,13 +278,9 @@ struct Shape {
 // 256 sets: 860).  The thread per set also takes targets of more repetitions
 // than a step's term buffer holds.
 inline Shape shape_for(const Args& a, int sms) {
+    if (a.REP > (uint32_t)TERMS / 4 || lane_us(a, sms) < cta_us(a, sms)) return {0, 0};
     const uint64_t words = (uint64_t)a.ns * a.so;
-    const uint32_t rows = a.samples ? a.p_rep : 1u;
-    if (a.REP > (uint32_t)TERMS / 4) return {0, 0};
-    const double lane_us = (double)words * (0.45 + 0.06 * rows);
-    const double cta_us = (double)a.nsets / sms * (0.85 + 0.0057 * (double)words);
-    if (rows <= 16u && lane_us < cta_us) return {0, 0};
-    if (words * rows < (1ull << 18)) return {1, 128};
+    if (words * (a.samples ? a.p_rep : 1u) < (1ull << 18)) return {1, 128};
     if (2ull * a.nsets <= (uint64_t)sms) return {1, 512};
     return {2, 128};
 }
