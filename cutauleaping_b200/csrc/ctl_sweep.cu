@@ -325,9 +325,9 @@ static ctl_status occupancy(int dev, const void* k, int threads, size_t smem, in
 // geometry as compile-time constants: species, reactions, tree leaves, sample
 // instants and sampled species.  Loops over a lane's leaves unroll and the
 // slots' offsets fold into the code; the tables stay in device memory
-// (dev::Tables, the same kernel parameter as the first part of dev::Model).  On the 64 x 128
-// network of the 65,536-simulation benchmark at 8 lanes per simulation this
-// takes a sweep from 1,672 to 1,232 ms on one B200, with identical bits.
+// (dev::Tables, the same kernel parameter as the first part of dev::Model).
+// 16,384 simulations of the 64 x 128 network to t 1 at 8 lanes each take 187 ms
+// with the library's kernel and 114 compiled on one B200, with identical bits.
 // Compiled once per process and (geometry, group size, register budget).
 
 // Batches of at least this many simulations use the compiled kernel when
@@ -469,9 +469,9 @@ static ctl_status plan_tiny(ctl_model* m, const ctl_run_cfg* cfg, uint32_t n, La
     pl.tinySM = tiny_species_bound(t);
     // register budget of the kernel compiled for the network (the library's
     // own is built for 2): 1 by default, which leaves the Schlogl kernels
-    // unspilled (254 registers for block rounds, 187 for warp lockstep,
-    // against 128 with spills at 2) -- 4,096 simulations on one B200: 330k
-    // against 295k sims/s; 65,536: 722k against 650k
+    // unspilled (239 registers for block rounds, 191 for warp lockstep,
+    // against 128 with spills at 2): 4,096 simulations to t 5 on one B200 8.9
+    // ms against 10.1; 65,536 27.1 against 25.5
     const int minb = cfg->min_blocks > 0 ? cfg->min_blocks : 1;
     const int sched = cfg->sched > 0 ? cfg->sched : tiny_sched(cfg, n, da.sm_count);
     pl.spec = cfg->spec >= 0 ? tiny_kernel_of(m, cfg->flags, minb, sched) : nullptr;
@@ -617,8 +617,12 @@ static ctl_status plan_launch(ctl_model* m, const ctl_run_cfg* cfg_in, uint32_t 
     pl.sched = cfg->sched > 0 ? cfg->sched : 1;
     int G = cfg->group > 0 ? cfg->group : heuristic_group(t);
     if (cfg->group <= 0) {
-        // small batches (fewer lanes than one 256-thread block per SM): more
-        // lanes per simulation so that every SM gets warps
+        // Small batches (fewer lanes than one 256-thread block per SM): more
+        // lanes per simulation so that every SM gets warps.  One B200, ms with
+        // 4, 8, 16 and 32 lanes: 12 x 20 exact, 500 simulations 22, 8.5, 8.6,
+        // 9.1; 2,000: 22, 8.9, 9.8, 10.8; 8,192 (8 taken): 19, 7.6, 20, 24.
+        // 64 x 128 to t 1, 500: 250, 90, 59, 37; 2,000: 258, 84, 60, 44; 5,000
+        // (8 taken): 100, 53, 65, 73.
         DevAttr da0;
         if (device_attr(cfg->device, da0) != CTL_OK) return CTL_ERR_CUDA;
         const int gmax = std::min(t.P, 32);

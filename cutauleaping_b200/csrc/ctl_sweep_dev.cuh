@@ -6,10 +6,11 @@
 // PreCalculations (2phase_n-tau-leaping.cu:1568-2093), EventualSSASteps
 // (2099-2273), LightweightSSA (2280-2454), setup_random (2974-2988),
 // PrepareVariables (1269-1297) and ParallelVoting (2990-3002) with ONE
-// launch: every group of G lanes owns a shared-memory slot, pulls a
-// simulation from a device work queue (atomic ticket), runs it to the end
-// (leaps, SSA bursts, samples) and pulls the next one.  No host round trip
-// per leap, no per-pass reload of state from global memory.
+// launch: blocks hold simulations in shared-memory slots, run each to the end
+// (leaps, SSA bursts, samples; a group of G lanes at a time, which need not be
+// the same one from one stretch of work to the next) and pull the next one from
+// a device work queue (atomic ticket).  No host round trip per leap, no per-pass
+// reload of state from global memory.
 //
 // Determinism contract (what makes any launch shape give identical bits):
 //   * every random word comes from Philox4x32-10 with key = seed and counter
@@ -562,7 +563,9 @@ __device__ __forceinline__ void finish_zero(const M& m, const Run& run, Slot<M> 
             for (int k = (int)lane; k < so; k += G) out.put(0u, so, k, (uint32_t)sl.x((int)m.cs[k]));
             cursor = 1;
         }
-        // each lane copies its own columns k, which it wrote itself
+        // the row copied forward may be another warp's: its writes lie before
+        // the fence with which that warp put the simulation back into the pool,
+        // these reads behind the one with which this warp took it
         for (uint32_t i = cursor; i < ns; i++)
             for (int k = (int)lane; k < so; k += G) out.put(i, so, k, out.get(cursor - 1, so, k));
     } else {
@@ -1157,9 +1160,10 @@ __device__ __forceinline__ void finish_sim(const Grp<G>& g, const M& m, const Ru
         run.info[sim] = inf;
     }
     if (run.out_host && out.samples) {
-        // the group's lanes wrote the rows; after the barrier every lane sees
-        // them and the group copies the simulation's row to the caller's
-        // pinned buffer (16-byte stores when the row allows)
+        // rows that this group wrote are visible to its lanes after the barrier,
+        // those of warps that held the simulation before by the pool's fences;
+        // the group copies them all to the caller's pinned buffer (16-byte
+        // stores when the row allows)
         g.sync();
         if (act) {
             const size_t words = (size_t)m.ns * (size_t)so;

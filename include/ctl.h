@@ -212,9 +212,10 @@ ctl_status ctl_spec_source(const ctl_model* m, int32_t group, int32_t min_blocks
  * memory (an application whose device memory comes only from its own pool,
  * a host that has fixed its device-memory budget, a layer that must not grow
  * memory behind its caller).  No counterpart in the reference.  The model
- * tables and the work-queue ticket live in a fixed 1 MiB array inside the
- * library instead of a cudaMalloc'd copy; models whose tables need more are
- * rejected with CTL_ERR_SHAPE.  The call allocates nothing: no cudaMalloc,
+ * tables and the work-queue ticket live in a fixed 4 MiB array inside the
+ * library instead of a cudaMalloc'd copy; models whose plain tables (one word
+ * per dependent reaction) need more than 1 MiB are rejected with
+ * CTL_ERR_SHAPE.  The call allocates nothing: no cudaMalloc,
  * no cudaFree, no allocating library routine.  The first call on a device
  * looks up the array's device address (make it before any stream capture).
  * Every call reuses the same array and leaves its contents behind, so calls
