@@ -315,33 +315,32 @@ struct Tree {
     double root;
 };
 
-// Chunk q's leaves.  Mode 0: propensities; 1: those of critical reactions
-// (whose am is 0, where the others' am is a copy of a); 2: as 1 but leaf 0
-// unmasked (the reference's critical pick, tau.cu:1997).
-template <class M>
+// Chunk q's leaves.  Mode 0: propensities; 1: those of critical reactions (whose
+// am is 0, where the others' am is a copy of a); 2: as 1 but leaf 0 unmasked (the
+// reference's critical pick, tau.cu:1997).  By a select, by the exclusive or of
+// the two words (0 for equal words, a against 0), or, FAST, by a - am, which is no
+// number where a non-critical propensity overflows FP32.  Groups of several
+// warps subtract and look again where that gives no number; exclusive ors take
+// the busier integer pipe there (512 x 1024 to t 0.06, 4,736 simulations: 528.6
+// against 537 ms).  In smaller groups the second look's code costs more (the
+// uneven batch: 344.0 against 332.9).
+constexpr int BY_SELECT = 0, BY_XOR = 1, FAST = 2;
+template <int G>
+constexpr int SOUND = G > 32 ? BY_SELECT : BY_XOR;
+template <int HOW, class M>
 __device__ __forceinline__ float4 leaves(const M& m, const Slot<M>& sl, int q, int mode) {
     float4 v = sl.chunk(m, q);
     if (mode) {
         const float4 n = reinterpret_cast<const float4*>(sl.am(m))[q];
-        v.x = n.x == 0.0f || (mode == 2 && q == 0) ? v.x : 0.0f;
-        v.y = n.y == 0.0f ? v.y : 0.0f;
-        v.z = n.z == 0.0f ? v.z : 0.0f;
-        v.w = n.w == 0.0f ? v.w : 0.0f;
-    }
-    return v;
-}
-// The same as a - am, a subtraction where a select or an exclusive or takes the
-// busier integer pipe (512 x 1024, 4,736 simulations to t 0.06: 527 against 537
-// ms with exclusive ors).  No number where a non-critical propensity overflows FP32.
-template <class M>
-__device__ __forceinline__ float4 leaves_fast(const M& m, const Slot<M>& sl, int q, int mode) {
-    float4 v = sl.chunk(m, q);
-    if (mode) {
-        const float4 n = reinterpret_cast<const float4*>(sl.am(m))[q];
-        v.x = mode == 2 && q == 0 ? v.x : v.x - n.x;
-        v.y = v.y - n.y;
-        v.z = v.z - n.z;
-        v.w = v.w - n.w;
+        auto critical = [](float a, float am) {
+            if constexpr (HOW == FAST) return a - am;
+            else if constexpr (HOW == BY_XOR) return __uint_as_float(__float_as_uint(a) ^ __float_as_uint(am));
+            else return am == 0.0f ? a : 0.0f;
+        };
+        v.x = mode == 2 && q == 0 ? v.x : critical(v.x, n.x);
+        v.y = critical(v.y, n.y);
+        v.z = critical(v.z, n.z);
+        v.w = critical(v.w, n.w);
     }
     return v;
 }
@@ -350,11 +349,11 @@ __device__ __forceinline__ double sum4(const float4& v) {
 }
 
 // Binary-tree sum of chunks [q, q + n), n a power of two.
-template <class M>
+template <int HOW, class M>
 __device__ __forceinline__ double range_sum(const M& m, Slot<M> sl, int q, int n, int mode) {
     double st[16];  // st[l]: a finished subtree of 2^l chunks
     for (int i = 0; i < n; i++) {
-        double v = sum4(leaves(m, sl, q + i, mode));
+        double v = sum4(leaves<HOW>(m, sl, q + i, mode));
         int l = 0;
         for (int b = i; b & 1; b >>= 1) v = st[l++] + v;
         st[l] = v;
@@ -369,7 +368,7 @@ __device__ __forceinline__ void tree_build(const Grp<G>& g, const M& m, const Sl
     constexpr int NC = Tree<G, M>::NC;
     if (nch <= NC) {
 #pragma unroll
-        for (int k = 0; k < NC; k++) t.c4[k] = k < nch && own ? sum4(leaves_fast(m, sl, q0 + k, mode)) : 0.0;
+        for (int k = 0; k < NC; k++) t.c4[k] = k < nch && own ? sum4(leaves<(G > 32 ? FAST : BY_XOR)>(m, sl, q0 + k, mode)) : 0.0;
         double v[NC];
         auto add_up = [&]() {
 #pragma unroll
@@ -380,14 +379,14 @@ __device__ __forceinline__ void tree_build(const Grp<G>& g, const M& m, const Sl
                 for (int k = 0; k < NC; k += 2 * w) v[k] = v[k] + v[k + w];
         };
         add_up();
-        if (mode && v[0] != v[0]) {  // an overflowed propensity less itself
+        if (G > 32 && mode && v[0] != v[0]) {  // an overflowed propensity less itself
 #pragma unroll
-            for (int k = 0; k < NC; k++) t.c4[k] = k < nch && own ? sum4(leaves(m, sl, q0 + k, mode)) : 0.0;
+            for (int k = 0; k < NC; k++) t.c4[k] = k < nch && own ? sum4(leaves<SOUND<G>>(m, sl, q0 + k, mode)) : 0.0;
             add_up();
         }
         t.tot = v[0];
     } else {
-        t.tot = range_sum(m, sl, q0, nch, mode);
+        t.tot = range_sum<SOUND<G>>(m, sl, q0, nch, mode);
     }
     double s = t.tot;
 #pragma unroll
@@ -475,13 +474,13 @@ __device__ __forceinline__ int descend(const Grp<G>& g, const M& m, const Slot<M
         }
     } else if (on) {
         for (int h = nch / 2; h > 0; h >>= 1) {
-            const double L = range_sum(m, sl, q0 + k, h, mode), R = range_sum(m, sl, q0 + k + h, h, mode);
+            const double L = range_sum<SOUND<G>>(m, sl, q0 + k, h, mode), R = range_sum<SOUND<G>>(m, sl, q0 + k + h, h, mode);
             if (go_right(x, L, R)) k += h;
         }
     }
     // a lane beyond the leaves (P < 4 G) is never on the path
     const int q = m.P >= 4 * G || (q0 + k) * 4 < m.P ? q0 + k : 0;
-    const float4 v = leaves(m, sl, q, mode);
+    const float4 v = leaves<SOUND<G>>(m, sl, q, mode);
     const double v0 = (double)v.x, v1 = (double)v.y, v2 = (double)v.z, v3 = (double)v.w;
     const bool h1 = go_right(x, v0 + v1, v2 + v3);
     const bool h2 = go_right(x, h1 ? v2 : v0, h1 ? v3 : v1);
